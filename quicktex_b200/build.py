@@ -35,7 +35,7 @@ LIB = os.path.join(HERE, "libquicktex_cuda.so")
 EXT = os.path.join(HERE, "_quicktex" + sysconfig.get_config_var("EXT_SUFFIX"))
 BLOB = os.path.join(HERE, "data", "bc1_order_tables.bin")
 
-KERNEL_SRCS = ["qt_kernels.cu", "qt_noalloc.cu", "qt_resize.cu"]
+KERNEL_SRCS = ["qt_kernels.cu", "qt_coop.cu", "qt_noalloc.cu", "qt_resize.cu"]
 HOST_SRCS = ["qt_capi.cpp", "qt_batch.cpp", "qt_server.cpp"]
 # every header a source may include: the kernels include qt_bc1_thread.cuh
 HEADERS = sorted(os.path.join(CSRC, f) for f in os.listdir(CSRC) if f.endswith((".h", ".cuh"))) + \
@@ -82,7 +82,7 @@ def build(force: bool = False, verbose: bool = False) -> None:
             # -fmad=false: no float multiply-add contraction anywhere, the reference's x86-64 SSE
             # arithmetic (one rounding per operation) whether or not an expression is written with
             # explicit round-to-nearest intrinsics
-            cmd = [NVCC, "-O3", "-std=c++17", *ARCH, "-lineinfo", "-fmad=false", "-Xcompiler", "-fPIC", "-I" + INCLUDE,
+            cmd = [NVCC, "-O3", "-std=c++17", *ARCH, "-lineinfo", "-fmad=false", "--split-compile", "0", "-Xcompiler", "-fPIC", "-I" + INCLUDE,
                    "-I" + CSRC, "-c", s, "-o", o]
             if verbose:
                 cmd.insert(1, "-Xptxas=-v")

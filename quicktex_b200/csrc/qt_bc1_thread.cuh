@@ -10,6 +10,12 @@
 // round-to-nearest intrinsics in the reference's operation order; every texel
 // sum is an exact integer.
 
+// Words between the rows of t_px beyond the threads: 1 puts the rows a bank apart, so that a warp reads one block's
+// texels (a column) without conflicts, as the cooperative kernels do; with 0, a row's address is a shift of its index.
+#ifndef QT_TEXEL_PAD
+#define QT_TEXEL_PAD 0
+#endif
+
 namespace tpb {
 
 constexpr int kThreads = 128;
@@ -22,10 +28,10 @@ constexpr int kThreads = 128;
 // Check2 L0 +2.5-4%, L10 +2-4.5%; Faster (which also selects among four errors instead of
 // among palette words) L5 +4.5-7%, L7 +12%, BC3 L5 +8%; FindSelectors' Full loop +1-2% at the
 // three-colour settings.
-__constant__ int kNeg2 = -2;
-__constant__ int kNeg1 = -1;
+static __constant__ int kNeg2 = -2;
+static __constant__ int kNeg1 = -1;
 
-__shared__ uint32_t t_px[16][kThreads];     // texel i of the thread's block
+__shared__ uint32_t t_px[16][kThreads + QT_TEXEL_PAD];  // texel i of the thread's block
 __shared__ uint32_t t_srg[17][kThreads];    // cluster-fit prefix sums: r | g << 16
 __shared__ uint16_t t_sb[17][kThreads];     //                          b
 
@@ -104,7 +110,7 @@ __device__ __forceinline__ M metrics_body(bool ignore_black) {
 // their instruction working set small when one kernel serves every setting; the specialised
 // kernels (k_bc1_fast: one selector kind, no EndpointSearch) inline the bodies, which saves
 // the call overhead where the per-block work is small. INL picks one at compile time.
-__device__ __noinline__ M metrics(bool ignore_black) { return metrics_body(ignore_black); }
+static __device__ __noinline__ M metrics(bool ignore_black) { return metrics_body(ignore_black); }
 template <bool INL> __device__ __forceinline__ M metrics_(bool ignore_black) {
     if constexpr (INL) return metrics_body(ignore_black);
     else return metrics(ignore_black);
@@ -487,7 +493,7 @@ __device__ __forceinline__ int2 find_endpoints_body(const M &m, int mode, bool i
     return make_int2(lo, hi);
 }
 
-__device__ __noinline__ int2 find_endpoints(const M &m, int mode, bool ignore_black, int power_iters) {
+static __device__ __noinline__ int2 find_endpoints(const M &m, int mode, bool ignore_black, int power_iters) {
     return find_endpoints_body(m, mode, ignore_black, power_iters);
 }
 template <bool INL> __device__ __forceinline__ int2 find_endpoints_(const M &m, int mode, bool ignore_black, int power_iters) {
@@ -1036,34 +1042,6 @@ __global__ void __launch_bounds__(256) k_bc1_split(const uint8_t *__restrict__ r
 // 24 → +2.5% at level 18 over refilling every lane as soon as it is idle)
 constexpr int kRefillBatch = 8;
 
-struct SearchQueues {
-    uint32_t *count;  // [3] entries per queue
-    uint32_t *head;   // [3] next entry to take
-    uint32_t *b, *lohi, *err, *sel, *mode;  // [3][cap] each
-    long cap;
-};
-
-// Searches that moved the endpoints, finished by k_bc1_finish: the block, its final endpoints
-// and colour mode. The reference keeps the selectors of the last accepted trial, which
-// FindSelectors computed from those endpoints (BC1Encoder.cpp:974-990); the search rounds here
-// compute errors only, so the selectors are computed once at the end. Done inside the refill loop,
-// that would run with one lane of the warp active.
-struct FinishQueue {
-    uint32_t *count;
-    uint32_t *b, *lohi, *mode;  // [cap] each
-};
-
-// Blocks whose EncodeBlock continues in k_bc1_cf2 after the first four-colour cluster-fit
-// pass (one entry per block: its index, the result after the first pass, the endpoints
-// before refinement). Entries that run the second pass fill the arrays from the front,
-// entries that only run the 3-colour trials from the back, so warps of k_bc1_cf2 see one
-// kind.
-struct Cf2Queue {
-    uint32_t *count;  // [2]: second-pass entries, 3-colour-only entries
-    uint32_t *b, *lohi, *err, *sel, *mode, *orig;  // [cap] each
-    long cap;
-};
-
 __device__ __forceinline__ uint32_t pack_lohi(const tpb::R &r) { return (uint32_t)r.lo | ((uint32_t)r.hi << 16); }
 
 // Appends the lanes' deferred searches to their queues (warp-aggregated). Every lane of
@@ -1084,6 +1062,30 @@ __device__ __forceinline__ void push_searches(const SearchQueues &q, const tpb::
             q.err[slot] = d.r.err;
             q.sel[slot] = d.r.sel;
             q.mode[slot] = (uint32_t)d.r.mode;
+        }
+    }
+}
+
+// Appends the lanes' blocks whose EncodeBlock continues in the second-pass kernel to its queue: those with a
+// second pass at the front, the others at the back. Every lane of the warp calls it.
+__device__ __forceinline__ void push_cf2(const Cf2Queue &c, const tpb::Deferred &d, long b, int lane) {
+#pragma unroll
+    for (int kind = 0; kind < 2; kind++) {
+        const bool mine = d.cf2 && d.pass2 == (kind == 0);
+        const uint32_t m = __ballot_sync(0xffffffffu, mine);
+        if (!m) continue;
+        uint32_t base = 0;
+        if (lane == 0) base = atomicAdd(c.count + kind, (uint32_t)__popc(m));
+        base = __shfl_sync(0xffffffffu, base, 0);
+        if (mine) {
+            const long idx = (long)base + __popc(m & ((1u << lane) - 1));
+            const long slot = kind == 0 ? idx : c.cap - 1 - idx;
+            c.b[slot] = (uint32_t)b;
+            c.lohi[slot] = pack_lohi(d.r);
+            c.err[slot] = d.r.err;
+            c.sel[slot] = d.r.sel;
+            c.mode[slot] = (uint32_t)d.r.mode;
+            c.orig[slot] = pack_lohi(d.orig);
         }
     }
 }
@@ -1144,25 +1146,7 @@ __global__ void __launch_bounds__(tpb::kThreads, 4) k_bc1_defer(const uint8_t *_
             }
         }
         push_searches(q, d, b, lane);
-#pragma unroll
-        for (int kind = 0; kind < 2; kind++) {
-            const bool mine = d.cf2 && d.pass2 == (kind == 0);
-            const uint32_t m = __ballot_sync(0xffffffffu, mine);
-            if (!m) continue;
-            uint32_t base = 0;
-            if (lane == 0) base = atomicAdd(c.count + kind, (uint32_t)__popc(m));
-            base = __shfl_sync(0xffffffffu, base, 0);
-            if (mine) {
-                const long idx = (long)base + __popc(m & ((1u << lane) - 1));
-                const long slot = kind == 0 ? idx : c.cap - 1 - idx;
-                c.b[slot] = (uint32_t)b;
-                c.lohi[slot] = pack_lohi(d.r);
-                c.err[slot] = d.r.err;
-                c.sel[slot] = d.r.sel;
-                c.mode[slot] = (uint32_t)d.r.mode;
-                c.orig[slot] = pack_lohi(d.orig);
-            }
-        }
+        push_cf2(c, d, b, lane);
     }
 }
 

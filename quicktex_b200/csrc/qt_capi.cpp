@@ -134,6 +134,40 @@ void build_factors(int n, int count, const uint8_t *hist, float (*fac)[4], uint1
     }
 }
 
+// The orderings as the cooperative cluster fit reads them, 16 bytes each: the factor matrix (symmetric:
+// its second and third entries are equal) and where the prefix sums of its selectors start.
+void build_ord(int n, int count, const uint8_t *hist, const float (*fac)[4], uint32_t (*ord)[4]) {
+    for (int i = 0; i < count; i++) {
+        const float f[3] = {fac[i][0], fac[i][1], fac[i][3]};
+        std::memcpy(ord[i], f, sizeof f);
+        uint32_t at = 0, packed = 0;
+        for (int s = 0; s < n - 1; s++) {
+            at += hist[(size_t)i * n + s];
+            packed |= (8 * at) << (8 * s);
+        }
+        ord[i][3] = packed;
+    }
+}
+
+// BestOrders for lanes that each take one of 32 consecutive entries (a warp's step) and read its ordering from
+// shared memory, 16 bytes at ordering * 16: a quarter-warp's eight reads go without bank conflicts when their
+// orderings differ modulo 8, so each 32 entries are dealt over the four quarter-warps that way. Each keeps its
+// place in the list.
+void build_coop(const uint16_t *best, size_t n, uint16_t *coop) {
+    for (size_t at = 0; at < n; at += 32) {
+        int used[4] = {0, 0, 0, 0}, same[4][8] = {};
+        for (int place = 0; place < 32; place++) {
+            const uint16_t e = best[at + place];
+            const int th = e & 0x7FFF, bank = th & 7;
+            int q = -1;
+            for (int k = 0; k < 4; k++)
+                if (used[k] < 8 && (q < 0 || same[k][bank] < same[q][bank] || (same[k][bank] == same[q][bank] && used[k] < used[q]))) q = k;
+            same[q][bank]++;
+            coop[at + 8 * q + used[q]++] = (uint16_t)(th | ((e & 0x8000) ? 0x400 : 0) | (place << 11));
+        }
+    }
+}
+
 qtk::HostTables *make_tables() {
     auto *t = new qtk::HostTables();
     std::memset(t, 0, sizeof *t);
@@ -154,6 +188,10 @@ qtk::HostTables *make_tables() {
     }
     build_factors(4, 969, o4, t->factors4, t->hash4, t->orders4);
     build_factors(3, 153, o3, t->factors3, t->hash3, t->orders3);
+    build_ord(4, 969, o4, t->factors4, t->ord4);
+    build_ord(3, 153, o3, t->factors3, t->ord3);
+    build_coop(t->best4, 969 * 128, t->coop4);
+    build_coop(t->best3, 153 * 32, t->coop3);
     for (int it = 0; it < 4; it++) {
         build_match(it, 5, t->match5[it]);
         build_match(it, 6, t->match6[it]);
