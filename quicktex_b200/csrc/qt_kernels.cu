@@ -35,7 +35,7 @@ namespace qtk {
 // 31 bits (the common case: no 64-bit division per block), else uint64_t. BC5 is held to
 // 40 registers (6 CTAs of 256 threads per SM instead of 5 at its natural 44): its loads
 // need the extra warps in flight (measured 0.83 -> 0.88 of HBM at 16384^2, bit-identical).
-// BC4 gives no minimum (0), where the compiler also settles at 40 registers; an explicit
+// BC4 gives no minimum (0), where the compiler settles at 32 registers; an explicit
 // minimum of 1 to 4 CTAs lets it take 52-56 and costs BC4 a tenth of its bandwidth.
 //
 // BC4: one block per thread. BC5 (two channels' arithmetic per texel) was latency-bound, so its
@@ -45,15 +45,16 @@ namespace qtk {
 // are conflict-free, and the block in flight holds no registers (0.88 -> 0.905 of HBM; the same
 // for BC4 measured 0.97 -> 0.91, so BC4 keeps the plain loop). Edge blocks of a texture whose
 // width is not a multiple of 4 (or an unaligned base) are loaded directly, with the wrap rule.
-template <bool BC5, typename Idx>
+template <bool BC5, typename Idx, bool STAGED = BC5>
 __global__ void __launch_bounds__(256, BC5 ? 6 : 0) k_bc4_encode(const uint8_t *__restrict__ rgba, int w, int h, Idx bw, Idx b_begin,
                                                     Idx nblocks, int c0, int c1, int aligned, uint8_t *__restrict__ out) {
-    if constexpr (!BC5) {
+    if constexpr (!STAGED) {
         for (Idx b = b_begin + (Idx)blockIdx.x * blockDim.x + threadIdx.x; b < nblocks; b += (Idx)gridDim.x * blockDim.x) {
             const int by = (int)(b / bw), bx = (int)(b - (Idx)by * bw);
             uint32_t px[16];
-            load_block_thread(rgba, w, h, bx, by, aligned && (bx * 4 + 4 <= w) && (by * 4 + 4 <= h), px);
-            reinterpret_cast<uint2 *>(out)[b] = bc4_block_thread(px, c0);
+            load_block_any(rgba, w, h, bx, by, aligned && (bx * 4 + 4 <= w) && (by * 4 + 4 <= h), px);
+            if constexpr (BC5) reinterpret_cast<uint4 *>(out)[b] = bc5_block_thread(px, c0, c1);
+            else reinterpret_cast<uint2 *>(out)[b] = bc4_block_thread(px, c0);
         }
         return;
     }
@@ -222,14 +223,22 @@ __device__ __forceinline__ void decode_texels(const uint8_t *__restrict__ blocks
 // is stored only if no later block (in the reference's by, bx, x, y write
 // order) writes the same wrapped position: source (px, py) is final iff
 // px + w >= 4*bw and py + h >= 4*bh (RawTexture::SetBlock, Texture.h:114-134).
+// An interior block of a texture whose rows are off the 16-byte grid stores its texels one by one at fixed offsets. The
+// wrapped form took all blocks of such a texture, two divisions a texel: BC1 8191 x 8190 162 -> 71 us, BC5 176 -> 73; aligned
+// words formed by shuffles across lanes: 83.
 __device__ __forceinline__ void store_block(const uint32_t px[16], int w, int h, int bw, int bh, int bx, int by,
                                             bool aligned, uint8_t *__restrict__ rgba) {
-    const bool interior = aligned && bx > 0 && by > 0 && bx * 4 + 4 <= w && by * 4 + 4 <= h;
-    if (interior) {
+    if (bx > 0 && by > 0 && bx * 4 + 4 <= w && by * 4 + 4 <= h) {
+        uint32_t *at = reinterpret_cast<uint32_t *>(rgba) + (size_t)(by * 4) * w + bx * 4;
 #pragma unroll
-        for (int y = 0; y < 4; y++)
-            *reinterpret_cast<uint4 *>(rgba + ((size_t)(by * 4 + y) * w + bx * 4) * 4) =
-                make_uint4(px[4 * y], px[4 * y + 1], px[4 * y + 2], px[4 * y + 3]);
+        for (int y = 0; y < 4; y++, at += w) {
+            if (aligned) {
+                *reinterpret_cast<uint4 *>(at) = make_uint4(px[4 * y], px[4 * y + 1], px[4 * y + 2], px[4 * y + 3]);
+            } else {
+#pragma unroll
+                for (int x = 0; x < 4; x++) at[x] = px[4 * y + x];
+            }
+        }
     } else {
 #pragma unroll
         for (int y = 0; y < 4; y++)
@@ -237,7 +246,7 @@ __device__ __forceinline__ void store_block(const uint32_t px[16], int w, int h,
             for (int x = 0; x < 4; x++) {
                 const int sx = bx * 4 + x, sy = by * 4 + y;
                 if (sx + w >= 4 * bw && sy + h >= 4 * bh)
-                    *reinterpret_cast<uint32_t *>(rgba + ((size_t)(sy % h) * w + (sx % w)) * 4) = px[4 * y + x];
+                    *reinterpret_cast<uint32_t *>(rgba + ((size_t)wrapped(sy, h) * w + wrapped(sx, w)) * 4) = px[4 * y + x];
             }
     }
 }
@@ -714,7 +723,7 @@ int launch_bc4_encode_range(const uint8_t *rgba, int w, int h, int c0, int c1, b
     int grid = 0;
     if (small_index(b_end, &grid)) {
         grid = (int)((b_end - b_begin + 255) / 256);
-        if (bc5) {  // persistent: at most the CTAs the SMs hold at once (each thread then loops,
+        if (bc5 && aligned) {  // persistent: at most the CTAs the SMs hold at once (each thread then loops,
                     // its next block's copies in flight while it encodes)
             static int resident = 0;
             if (resident <= 0) {  // 32 KB of staging per CTA: the shared-memory carveout that fits 6
@@ -728,7 +737,9 @@ int launch_bc4_encode_range(const uint8_t *rgba, int w, int h, int c0, int c1, b
             grid = std::min(grid, resident);
         }
         const uint32_t ubw = (uint32_t)bw, u0 = (uint32_t)b_begin, un = (uint32_t)b_end;
-        if (bc5) k_bc4_encode<true, uint32_t><<<grid, 256, 0, s>>>(rgba, w, h, ubw, u0, un, c0, c1, aligned, out);
+        // rows off the 16-byte grid have nothing to stage: one block per thread (8190 x 8191: 66 us, persistent 85)
+        if (bc5 && !aligned) k_bc4_encode<true, uint32_t, false><<<grid, 256, 0, s>>>(rgba, w, h, ubw, u0, un, c0, c1, 0, out);
+        else if (bc5) k_bc4_encode<true, uint32_t><<<grid, 256, 0, s>>>(rgba, w, h, ubw, u0, un, c0, c1, aligned, out);
         else k_bc4_encode<false, uint32_t><<<grid, 256, 0, s>>>(rgba, w, h, ubw, u0, un, c0, c1, aligned, out);
     } else {
         const uint64_t ubw = (uint64_t)bw, u0 = (uint64_t)b_begin, un = (uint64_t)b_end;
