@@ -2,13 +2,15 @@
 // include/quicktex_cuda.h).
 //
 // A qt_batch owns, per device: the device work queue (texture descriptors,
-// tiles, and a two-word control block: queue head and tile count), pinned
-// host staging for it, and a CUDA graph holding the persistent kernel launch.
-// Every qt_batch_run cuts the textures into tiles (tile size per format/level
-// from the tuning rules), orders the tiles by estimated cost, heaviest first
-// (so the long L18 tiles start early and the cheap ones fill the tail),
-// uploads the queue, and replays the graph. The graph is re-captured only
-// when a queue buffer has to grow.
+// tiles, and a four-word control block: head and end of each of two tile
+// ranges), pinned host staging for it, and a CUDA graph holding the persistent
+// launch. Every qt_batch_run cuts the textures into tiles (tile size per
+// format/level from the tuning rules), orders the tiles by estimated cost,
+// heaviest first (so the long tiles start early and the cheap ones fill the
+// tail), uploads the queue, and replays the graph. The tiles of textures whose
+// cluster fit runs cooperatively (qt_bc1_coop.cuh: levels 16-19) go to a
+// kernel of their own beside k_batch, in the same graph. Graphs are
+// re-captured only when a queue buffer has to grow.
 
 #include <algorithm>
 #include <cstdlib>
@@ -72,9 +74,9 @@ struct qt_batch {
     uint32_t *d_ctl = nullptr, *h_ctl = nullptr;
     cudaEvent_t staged = nullptr;     // the last upload from the pinned staging buffers
     cudaEvent_t done = nullptr;       // the last persistent launch (the queue is in use until then)
-    cudaStream_t capture = nullptr;   // private stream the graph is captured on
-    cudaGraph_t graph = nullptr;
-    cudaGraphExec_t exec = nullptr;
+    cudaStream_t capture[2] = {};     // private streams the graphs are captured on: the cooperative kernel's, k_batch's
+    cudaEvent_t fork = nullptr, join = nullptr;
+    cudaGraphExec_t exec[4] = {};     // by what a run holds: 1 tiles of k_batch, 2 of the cooperative kernel, 3 both
 
     qt_batch() {
         for (int op = 0; op < 2; op++)
@@ -96,11 +98,18 @@ struct qt_batch {
 
 namespace {
 
+// the queue's smallest capacity: a run's tiles are cut finer to fill the GPU only while they fit it
+constexpr size_t kMinTiles = 16384;
+
+void drop_graphs(qt_batch *b) {
+    for (cudaGraphExec_t &e : b->exec) {
+        if (e) cudaGraphExecDestroy(e);
+        e = nullptr;
+    }
+}
+
 void free_buffers(qt_batch *b) {
-    if (b->exec) cudaGraphExecDestroy(b->exec);
-    if (b->graph) cudaGraphDestroy(b->graph);
-    b->exec = nullptr;
-    b->graph = nullptr;
+    drop_graphs(b);
     cudaFree(b->d_items);
     cudaFree(b->d_tiles);
     cudaFreeHost(b->h_items);
@@ -115,7 +124,7 @@ int grow(qt_batch *b, size_t items, size_t tiles) {
     if (b->staged) cudaEventSynchronize(b->staged);
     cudaDeviceSynchronize();  // the old queue may still be read by a running launch
     const size_t ni = std::max(items, std::max<size_t>(b->cap_items * 2, 64));
-    const size_t nt = std::max(tiles, std::max<size_t>(b->cap_tiles * 2, 1024));
+    const size_t nt = std::max(tiles, std::max<size_t>(b->cap_tiles * 2, kMinTiles));
     free_buffers(b);
     cudaError_t e;
     if ((e = cudaMalloc(&b->d_items, ni * sizeof(qtk::BatchItemDev))) != cudaSuccess ||
@@ -128,6 +137,34 @@ int grow(qt_batch *b, size_t items, size_t tiles) {
     }
     b->cap_items = ni;
     b->cap_tiles = nt;
+    return QT_OK;
+}
+
+// Captures a run's launches once (replays read the queue through fixed pointers): k_batch (kind 1), the cooperative
+// kernel (2) or both side by side (3).
+int capture(qt_batch *b, int kind) {
+    const int grid = b->ctas_per_sm > 0 ? qtk::batch_sms() * b->ctas_per_sm : 0;
+    cudaError_t e = cudaStreamBeginCapture(b->capture[0], cudaStreamCaptureModeThreadLocal);
+    if (e != cudaSuccess) return qtk::cuda_error((int)e, "graph capture");
+    int lrc = 0;
+    if (kind == 3 && (e = cudaEventRecord(b->fork, b->capture[0])) == cudaSuccess) e = cudaStreamWaitEvent(b->capture[1], b->fork, 0);
+    if (e == cudaSuccess && (kind & 2)) lrc = qtk::launch_batch_coop(b->d_items, b->d_tiles, b->d_ctl, b->capture[0]);
+    if (e == cudaSuccess && !lrc && (kind & 1))
+        lrc = qtk::launch_batch(b->d_items, b->d_tiles, b->d_ctl, grid, b->threads, b->capture[kind == 3]);
+    if (e == cudaSuccess && kind == 3 && (e = cudaEventRecord(b->join, b->capture[1])) == cudaSuccess)
+        e = cudaStreamWaitEvent(b->capture[0], b->join, 0);
+    cudaGraph_t g = nullptr;
+    const cudaError_t end = cudaStreamEndCapture(b->capture[0], &g);
+    if (lrc || e != cudaSuccess || end != cudaSuccess) {
+        if (g) cudaGraphDestroy(g);
+        return lrc ? qtk::cuda_error(lrc, "batch launch") : qtk::cuda_error((int)(e != cudaSuccess ? e : end), "graph capture");
+    }
+    e = cudaGraphInstantiate(&b->exec[kind], g, 0);
+    cudaGraphDestroy(g);
+    if (e != cudaSuccess) {
+        b->exec[kind] = nullptr;
+        return qtk::cuda_error((int)e, "graph instantiate");
+    }
     return QT_OK;
 }
 
@@ -170,9 +207,13 @@ int qt_batch_create(int device, qt_batch **out) {
         b->device = device;
         if ((e = cudaEventCreateWithFlags(&b->staged, cudaEventDisableTiming)) != cudaSuccess ||
             (e = cudaEventCreateWithFlags(&b->done, cudaEventDisableTiming)) != cudaSuccess ||
-            (e = cudaStreamCreateWithFlags(&b->capture, cudaStreamNonBlocking)) != cudaSuccess ||
-            (e = cudaMalloc(&b->d_ctl, 2 * sizeof(uint32_t))) != cudaSuccess ||
-            (e = cudaHostAlloc((void **)&b->h_ctl, 2 * sizeof(uint32_t), cudaHostAllocDefault)) != cudaSuccess) {
+            (e = cudaEventCreateWithFlags(&b->fork, cudaEventDisableTiming)) != cudaSuccess ||
+            (e = cudaEventCreateWithFlags(&b->join, cudaEventDisableTiming)) != cudaSuccess ||
+            // the cooperative kernel's node carries its stream's priority: its tiles, the long ones, start first
+            (e = cudaStreamCreateWithPriority(&b->capture[0], cudaStreamNonBlocking, -1)) != cudaSuccess ||
+            (e = cudaStreamCreateWithPriority(&b->capture[1], cudaStreamNonBlocking, 0)) != cudaSuccess ||
+            (e = cudaMalloc(&b->d_ctl, 4 * sizeof(uint32_t))) != cudaSuccess ||
+            (e = cudaHostAlloc((void **)&b->h_ctl, 4 * sizeof(uint32_t), cudaHostAllocDefault)) != cudaSuccess) {
             rc = qtk::cuda_error((int)e, "creating a batch");
             qt_batch_destroy(b);
             b = nullptr;
@@ -194,7 +235,10 @@ int qt_batch_destroy(qt_batch *b) {
     cudaFreeHost(b->h_ctl);
     if (b->staged) cudaEventDestroy(b->staged);
     if (b->done) cudaEventDestroy(b->done);
-    if (b->capture) cudaStreamDestroy(b->capture);
+    if (b->fork) cudaEventDestroy(b->fork);
+    if (b->join) cudaEventDestroy(b->join);
+    for (cudaStream_t s : b->capture)
+        if (s) cudaStreamDestroy(s);
     cudaSetDevice(prev);
     delete b;
     return QT_OK;
@@ -218,12 +262,7 @@ int qt_batch_set_rules(qt_batch *b, const qt_tile_rule *rules, size_t n) {
 int qt_batch_set_grid(qt_batch *b, int ctas_per_sm) {
     if (!b || ctas_per_sm < 0) return qtk::set_error(QT_ERR_ARG, "invalid grid");
     std::lock_guard<std::mutex> lk(b->mu);
-    if (ctas_per_sm != b->ctas_per_sm && b->exec) {
-        cudaGraphExecDestroy(b->exec);
-        cudaGraphDestroy(b->graph);
-        b->exec = nullptr;
-        b->graph = nullptr;
-    }
+    if (ctas_per_sm != b->ctas_per_sm) drop_graphs(b);
     b->ctas_per_sm = ctas_per_sm;
     return QT_OK;
 }
@@ -232,12 +271,7 @@ int qt_batch_set_threads(qt_batch *b, int threads_per_cta) {
     if (!b || (threads_per_cta != 32 && threads_per_cta != 64 && threads_per_cta != 128))
         return qtk::set_error(QT_ERR_ARG, "threads per CTA must be 32, 64 or 128");
     std::lock_guard<std::mutex> lk(b->mu);
-    if (threads_per_cta != b->threads && b->exec) {
-        cudaGraphExecDestroy(b->exec);
-        cudaGraphDestroy(b->graph);
-        b->exec = nullptr;
-        b->graph = nullptr;
-    }
+    if (threads_per_cta != b->threads) drop_graphs(b);
     b->threads = threads_per_cta;
     return QT_OK;
 }
@@ -273,13 +307,15 @@ int qt_batch_run(qt_batch *b, const qt_batch_item *items, size_t n, void *stream
     if (cur != b->device) return qtk::set_error(QT_ERR_STATE, "qt_batch_run: the batch belongs to another device");
     if (int rc = qtk::ensure_current_device(nullptr)) return rc;
 
-    // descriptors, and tiles ordered heaviest first
+    // descriptors, and each item's rule and kernel
     std::vector<qtk::BatchItemDev> dev(n);
-    struct Tile {
-        float cost;
-        qtk::TileDev t;
+    struct Plan {
+        Rule rule;
+        bool coop;
     };
-    std::vector<Tile> tiles;
+    std::vector<Plan> plan(n);
+    double work[2] = {0, 0};  // of k_batch, of the cooperative kernel
+    size_t coarse = 0;
     for (size_t i = 0; i < n; i++) {
         const qt_batch_item &it = items[i];
         if (int rc = check_item(it)) return rc;
@@ -300,13 +336,42 @@ int qt_batch_run(qt_batch *b, const qt_batch_item *items, size_t n, void *stream
         const uint64_t nb = (uint64_t)d.bw * d.bh;
         if (nb > 0xFFFFFFFFull) return qtk::set_error(QT_ERR_ARG, "Texture too large");
         const bool leveled = it.op == QT_OP_ENCODE && (it.format == 1 || it.format == 3);
-        const Rule &r = b->rules[rule_index(it.op, it.format, leveled ? qtk_level_of(it.params) : 0)];
-        for (uint64_t s0 = 0; s0 < nb; s0 += r.tile_blocks) {
-            const uint32_t cnt = (uint32_t)std::min<uint64_t>(r.tile_blocks, nb - s0);
-            tiles.push_back({r.cost * cnt, {(uint32_t)i, (uint32_t)s0, cnt, 0u}});
+        Plan &pl = plan[i];
+        pl.rule = b->rules[rule_index(it.op, it.format, leveled ? qtk_level_of(it.params) : 0)];
+        pl.coop = leveled && qtk::coop_batch_setting(it.params);
+        work[pl.coop] += (double)pl.rule.cost * (double)nb;
+        coarse += (size_t)((nb + pl.rule.tile_blocks - 1) / pl.rule.tile_blocks);
+    }
+    // Tiles of the rules' sizes, or smaller where a kernel's resident warps would have fewer than four each (a short
+    // batch waits for its longest tile): a cooperative warp works on one block at a time, so its tiles may fall to a few
+    // blocks; k_batch's keep 32, a block per lane.
+    const double warps[2] = {(double)qtk::batch_sms() * 16, (double)qtk::batch_coop_warps()};
+    const size_t finer = 4 * (size_t)(warps[0] + warps[1]) + n;
+    const bool cut = coarse + finer <= std::max(b->cap_tiles, kMinTiles);
+    struct Tile {
+        float cost;
+        qtk::TileDev t;
+    };
+    std::vector<Tile> tiles, rest;  // of the cooperative kernel, of k_batch; heaviest first
+    for (size_t i = 0; i < n; i++) {
+        const Plan &pl = plan[i];
+        const uint64_t nb = (uint64_t)dev[i].bw * dev[i].bh;
+        uint64_t tb = pl.rule.tile_blocks;
+        if (cut) {
+            const uint64_t fill = (uint64_t)(work[pl.coop] / (warps[pl.coop] * 4) / pl.rule.cost) + 1;
+            tb = std::min(tb, pl.coop ? fill : (fill + 31) / 32 * 32);
+        }
+        std::vector<Tile> &to = pl.coop ? tiles : rest;
+        for (uint64_t s0 = 0; s0 < nb; s0 += tb) {
+            const uint32_t cnt = (uint32_t)std::min<uint64_t>(tb, nb - s0);
+            to.push_back({pl.rule.cost * cnt, {(uint32_t)i, (uint32_t)s0, cnt, 0u}});
         }
     }
-    std::stable_sort(tiles.begin(), tiles.end(), [](const Tile &a, const Tile &c) { return a.cost > c.cost; });
+    const auto heavier = [](const Tile &a, const Tile &c) { return a.cost > c.cost; };
+    std::stable_sort(tiles.begin(), tiles.end(), heavier);
+    std::stable_sort(rest.begin(), rest.end(), heavier);
+    const size_t ncoop = tiles.size();
+    tiles.insert(tiles.end(), rest.begin(), rest.end());
     b->last_tiles = tiles.size();
     if (tiles.size() > 0xFFFFFFFFull) return qtk::set_error(QT_ERR_ARG, "too many tiles");
     if (tiles.empty()) return QT_OK;
@@ -316,37 +381,23 @@ int qt_batch_run(qt_batch *b, const qt_batch_item *items, size_t n, void *stream
     if (e != cudaSuccess) return qtk::cuda_error((int)e, "batch staging");
     std::memcpy(b->h_items, dev.data(), n * sizeof(qtk::BatchItemDev));
     for (size_t i = 0; i < tiles.size(); i++) b->h_tiles[i] = tiles[i].t;
-    b->h_ctl[0] = 0;
+    b->h_ctl[0] = (uint32_t)ncoop;  // k_batch's tiles follow the cooperative kernel's
     b->h_ctl[1] = (uint32_t)tiles.size();
+    b->h_ctl[2] = 0;
+    b->h_ctl[3] = (uint32_t)ncoop;
     cudaStream_t s = (cudaStream_t)stream;
     // runs on other streams: do not overwrite the queue before the previous launch finished reading it
     if ((e = cudaStreamWaitEvent(s, b->done, 0)) != cudaSuccess) return qtk::cuda_error((int)e, "batch ordering");
     if ((e = cudaMemcpyAsync(b->d_items, b->h_items, n * sizeof(qtk::BatchItemDev), cudaMemcpyHostToDevice, s)) != cudaSuccess ||
         (e = cudaMemcpyAsync(b->d_tiles, b->h_tiles, tiles.size() * sizeof(qtk::TileDev), cudaMemcpyHostToDevice, s)) != cudaSuccess ||
-        (e = cudaMemcpyAsync(b->d_ctl, b->h_ctl, 2 * sizeof(uint32_t), cudaMemcpyHostToDevice, s)) != cudaSuccess ||
+        (e = cudaMemcpyAsync(b->d_ctl, b->h_ctl, 4 * sizeof(uint32_t), cudaMemcpyHostToDevice, s)) != cudaSuccess ||
         (e = cudaEventRecord(b->staged, s)) != cudaSuccess)
         return qtk::cuda_error((int)e, "batch upload");
 
-    if (!b->exec) {  // capture the persistent launch once; replays read the queue through fixed pointers
-        const int grid = b->ctas_per_sm > 0 ? qtk::batch_sms() * b->ctas_per_sm : 0;
-        if ((e = cudaStreamBeginCapture(b->capture, cudaStreamCaptureModeThreadLocal)) != cudaSuccess)
-            return qtk::cuda_error((int)e, "graph capture");
-        const int lrc = qtk::launch_batch(b->d_items, b->d_tiles, b->d_ctl, grid, b->threads, b->capture);
-        cudaGraph_t g = nullptr;
-        e = cudaStreamEndCapture(b->capture, &g);
-        if (lrc != 0) {
-            if (g) cudaGraphDestroy(g);
-            return qtk::cuda_error(lrc, "batch launch");
-        }
-        if (e != cudaSuccess) return qtk::cuda_error((int)e, "graph capture");
-        if ((e = cudaGraphInstantiate(&b->exec, g, 0)) != cudaSuccess) {
-            cudaGraphDestroy(g);
-            b->exec = nullptr;
-            return qtk::cuda_error((int)e, "graph instantiate");
-        }
-        b->graph = g;
-    }
-    if ((e = cudaGraphLaunch(b->exec, s)) != cudaSuccess) return qtk::cuda_error((int)e, "graph launch");
+    const int kind = (ncoop < tiles.size() ? 1 : 0) | (ncoop ? 2 : 0);
+    if (!b->exec[kind])
+        if (int rc = capture(b, kind)) return rc;
+    if ((e = cudaGraphLaunch(b->exec[kind], s)) != cudaSuccess) return qtk::cuda_error((int)e, "graph launch");
     if ((e = cudaEventRecord(b->done, s)) != cudaSuccess) return qtk::cuda_error((int)e, "graph launch");
     return QT_OK;
 }

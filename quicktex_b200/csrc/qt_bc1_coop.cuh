@@ -32,7 +32,7 @@ struct Work {  // per CTA: what every cooperative kernel needs
 };
 struct FitWork {  // the cluster fit's on top
     uint2 pre[kWarps][32][17];   // prefix sums of a lane's block in rank order: r | g << 16, b
-    uint2 rnd5[32], rnd6[64];    // PreciseRound565: midpoint, then bytes: 8-bit values of r and r + 1, then r and r + 1 (Nvidia) or 0x66
+    uint2 rnd5[32], rnd6[64];    // PreciseRound565: midpoint, then bytes: 8-bit values of r and r + 1, 0x66
     uint4 ord4[969], ord3[153];  // per ordering: LS factors x, y (= z), w and the byte offsets of its three prefix sums
 };
 constexpr size_t kSearchSmem = sizeof(Work), kFitSmem = sizeof(Work) + sizeof(FitWork);
@@ -43,14 +43,14 @@ __device__ __forceinline__ FitWork &fit() { return *reinterpret_cast<FitWork *>(
 __device__ __forceinline__ uint32_t smem_addr(const void *p) { return (uint32_t)__cvta_generic_to_shared(p); }
 
 // fills the CTA's tables (every thread calls it; ends with a barrier)
-template <int IT> __device__ __forceinline__ void load_fit_tables(bool three) {
+__device__ __forceinline__ void load_fit_tables(bool three) {
     FitWork &F = fit();
     for (int i = threadIdx.x; i < 969; i += blockDim.x) F.ord4[i] = g_tab.ord4[i];
     if (three)
         for (int i = threadIdx.x; i < 153; i += blockDim.x) F.ord3[i] = g_tab.ord3[i];
     for (int i = threadIdx.x; i < 64; i += blockDim.x) {
-        if (i < 32) F.rnd5[i] = make_uint2(__float_as_uint(c_mid5[i]), (uint32_t)(s5to8(i) | ((s5to8(i + 1) & 0xFF) << 8)) | (IT == IT_NVIDIA ? (uint32_t)((i << 16) | ((i + 1) << 24)) : 0x660000u));
-        F.rnd6[i] = make_uint2(__float_as_uint(c_mid6[i]), (uint32_t)(s6to8(i) | ((s6to8(i + 1) & 0xFF) << 8)) | (IT == IT_NVIDIA ? (uint32_t)((i << 16) | ((i + 1) << 24)) : 0x660000u));
+        if (i < 32) F.rnd5[i] = make_uint2(__float_as_uint(c_mid5[i]), (uint32_t)(s5to8(i) | ((s5to8(i + 1) & 0xFF) << 8)) | 0x660000u);
+        F.rnd6[i] = make_uint2(__float_as_uint(c_mid6[i]), (uint32_t)(s6to8(i) | ((s6to8(i + 1) & 0xFF) << 8)) | 0x660000u);
     }
     __syncthreads();
 }
@@ -228,7 +228,7 @@ template <int IT, bool THREE> struct Palette {
 #pragma unroll
             for (int i = 0; i < 6; i++) {
                 v8[i] = (int)__byte_perm(w[i], 0u, up[i] ? 0x4441u : 0x4440u);
-                v5[i] = (int)__byte_perm(w[i], 0u, up[i] ? 0x4443u : 0x4442u);
+                v5[i] = v8[i] >> (i % 3 == 1 ? 2 : 3);  // the expansion keeps the value in its high bits
             }
             colour_row(rgb0(v8[0], v8[1], v8[2]), x.rg[0], x.b[0], x.n[0]);
             if (THREE) {
@@ -280,7 +280,8 @@ template <int IT, int K>
 __device__ __noinline__ void cluster_fit(const qt_bc1_params &p, bool run, tpb::R &r, const tpb::M &m, int pp_sum, int passes, bool *again) {
     constexpr bool four = !kind_three(K);
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, col0 = threadIdx.x - lane;
-    const unsigned total = p.exhaustive ? (four ? 969u : 153u) : (four ? p.orderings4 : p.orderings3);
+    const bool exhaustive = p.exhaustive != 0;
+    const unsigned total = exhaustive ? (four ? 969u : 153u) : (four ? p.orderings4 : p.orderings3);
     FitWork &F = fit();
     const uint4 *ord = four ? F.ord4 : F.ord3;
     const uint32_t tab5 = smem_addr(F.rnd5) - 8u * 0x4B000000u, tab6 = smem_addr(F.rnd6) - 8u * 0x4B000000u;
@@ -339,7 +340,7 @@ __device__ __noinline__ void cluster_fit(const qt_bc1_params &p, bool run, tpb::
             // a step's entry is loaded a step ahead
             auto entry = [&](unsigned q0) -> unsigned {
                 const unsigned q = q0 + lane;
-                if (!p.exhaustive) return q0 < total ? (unsigned)row[q0] : 0u;
+                if (!exhaustive) return q0 < total ? (unsigned)row[q0] : 0u;
                 return (q < total ? q : 0u) | (is_single_hash(four, (int)q) ? 0x400u : 0u) | ((unsigned)lane << 11);
             };
             unsigned next = entry(0);
@@ -393,8 +394,8 @@ __device__ __noinline__ void cluster_fit(const qt_bc1_params &p, bool run, tpb::
         }
         __syncwarp();
         if (won) {  // the winning trial's endpoints and selectors
-            const int raw = p.exhaustive ? (int)won_q : (int)(four ? g_tab.best4[start * 128 + won_q] : g_tab.best3[start * 32 + won_q]), th = raw & 0x7FFF;
-            if (p.exhaustive ? is_single_hash(four, th) : raw >= 0x8000) {
+            const int raw = exhaustive ? (int)won_q : (int)(four ? g_tab.best4[start * 128 + won_q] : g_tab.best3[start * 32 + won_q]), th = raw & 0x7FFF;
+            if (exhaustive ? is_single_hash(four, th) : raw >= 0x8000) {
                 r = sc;
             } else {
                 const uint4 o = ord[th];
@@ -699,7 +700,7 @@ __global__ void __launch_bounds__(tpb::kThreads, 4) k_bc1_coop(const uint8_t *__
                                                                 const uint32_t *__restrict__ list, const uint32_t *__restrict__ count, int per_warp) {
     load_tables_smem();
     const int color_mode = bc3 ? CM_FOUR : p.color_mode;  // BC3Encoder.h:39-40
-    coop::load_fit_tables<IT>(color_mode != CM_FOUR);
+    coop::load_fit_tables(color_mode != CM_FOUR);
     const int lane = threadIdx.x & 31;
     const long end = list ? (long)*count : nblocks, stride = (long)gridDim.x * coop::kWarps * per_warp;
     for (long wb = (list ? 0 : b_begin) + ((long)blockIdx.x * coop::kWarps + (threadIdx.x >> 5)) * per_warp; wb < end; wb += stride) {
@@ -727,7 +728,7 @@ __global__ void __launch_bounds__(tpb::kThreads, 4) k_bc1_coop_defer(const uint8
                                                                       SearchQueues q, Cf2Queue c) {
     load_tables_smem();
     const int color_mode = bc3 ? CM_FOUR : p.color_mode;  // BC3Encoder.h:39-40
-    coop::load_fit_tables<IT>(color_mode != CM_FOUR);
+    coop::load_fit_tables(color_mode != CM_FOUR);
     const int lane = threadIdx.x & 31;
     const long end = (long)*count, stride = (long)gridDim.x * blockDim.x;
     for (long wb = (long)blockIdx.x * blockDim.x + threadIdx.x - lane; wb < end; wb += stride) {
@@ -783,7 +784,7 @@ __global__ void __launch_bounds__(tpb::kThreads, 4) k_bc1_coop_cf2(const uint8_t
                                                                     uint8_t *__restrict__ out, int bc3, int aligned, Cf2Queue c, SearchQueues q) {
     load_tables_smem();
     const int color_mode = bc3 ? CM_FOUR : p.color_mode;
-    coop::load_fit_tables<IT>(color_mode != CM_FOUR);
+    coop::load_fit_tables(color_mode != CM_FOUR);
     const int lane = threadIdx.x & 31;
     const long n2 = (long)c.count[0], end = n2 + (long)c.count[1], stride = (long)gridDim.x * blockDim.x;
     for (long wb = (long)blockIdx.x * blockDim.x + threadIdx.x - lane; wb < end; wb += stride) {
@@ -882,4 +883,48 @@ __global__ void __launch_bounds__(tpb::kThreads, kCoopSearchCtas) k_bc1_coop_sea
     coop_search_queue<IT, K_F4_FULL>(0, rgba, w, h, bw, p.search_rounds, out, bc3, aligned, q, f);
     coop_search_queue<IT, K_T3>(1, rgba, w, h, bw, p.search_rounds, out, bc3, aligned, q, f);
     coop_search_queue<IT, K_TB>(2, rgba, w, h, bw, p.search_rounds, out, bc3, aligned, q, f);
+}
+
+// The batch's tiles whose textures run cooperatively (coop_batch_setting): tiles[0 .. ctl[3]), claimed through ctl[2] as
+// k_batch claims the others. One texture per tile, so a warp's settings are uniform.
+template <int IT> __device__ __noinline__ uint2 encode_warp_batch(const qt_bc1_params &p, int color_mode, bool have, int pp) {
+    return coop::encode_warp<IT>(p, color_mode, have, pp);
+}
+
+__global__ void __launch_bounds__(tpb::kThreads, 4) k_batch_coop(const BatchItemDev *__restrict__ items, const TileDev *__restrict__ tiles,
+                                                                 uint32_t *__restrict__ ctl) {
+    load_tables_smem();
+    coop::load_fit_tables(true);
+    const int lane = threadIdx.x & 31;
+    const uint32_t ntiles = ctl[3];
+    while (true) {
+        uint32_t t = 0;
+        if (lane == 0) t = atomicAdd(&ctl[2], 1u);
+        t = __shfl_sync(0xFFFFFFFFu, t, 0);
+        if (t >= ntiles) break;
+        const TileDev T = tiles[t];
+        const BatchItemDev &I = items[T.item];
+        const qt_bc1_params p = I.p;
+        const int bc3 = I.fmt == 3, w = I.w, h = I.h, cm = bc3 ? CM_FOUR : p.color_mode;  // BC3Encoder.h:39-40
+        const int aligned = ((w & 3) == 0) && ((reinterpret_cast<uintptr_t>(I.src) & 15) == 0);
+        for (uint32_t k = 0; k < T.count; k += 32) {
+            const bool have = k + lane < T.count;
+            const long b = (long)T.start + k + lane;
+            int pp = 0;
+            if (have) {
+                uint32_t v[16];
+                pp = stage_block(I.src, w, h, I.bw, b, aligned, v);
+            }
+            __syncwarp();
+            uint2 blk;
+            switch (p.interpolator) {
+                case IT_IDEAL: blk = encode_warp_batch<IT_IDEAL>(p, cm, have, pp); break;
+                case IT_ROUND: blk = encode_warp_batch<IT_ROUND>(p, cm, have, pp); break;
+                case IT_NVIDIA: blk = encode_warp_batch<IT_NVIDIA>(p, cm, have, pp); break;
+                default: blk = encode_warp_batch<IT_AMD>(p, cm, have, pp); break;
+            }
+            if (have) coop::write_out(I.dst, bc3, b, blk);
+            __syncwarp();
+        }
+    }
 }

@@ -38,6 +38,14 @@ bool coop_setting(const qt_bc1_params &p, long n) {
     return n <= (nvidia ? 3000 : 5000);
 }
 
+// The same for a texture of a batch, which shares full lanes with the others, and whose alternative (k_batch) runs the
+// second pass and the search on the lanes that need them.
+bool coop_batch_setting(const qt_bc1_params &p) {
+    if (p.error_mode != EM_FULL || p.search_rounds == 0) return false;
+    const unsigned trials = (p.exhaustive ? 969u : p.orderings4) * (p.two_cf_passes ? 2u : 1u);
+    return trials >= (p.interpolator == IT_NVIDIA ? 200u : 72u);
+}
+
 // Lets a cooperative kernel have its dynamic shared memory (above 48 KB with the static part); once per
 // kernel and device.
 template <typename K> static cudaError_t allow_smem(K kernel, size_t bytes, std::atomic<uint64_t> &done) {
@@ -112,6 +120,16 @@ void coop_defer_rest(const uint8_t *rgba, int w, int h, const qt_bc1_params &p, 
         k_bc1_coop_search<IT><<<num_sms() * kCoopSearchCtas, tpb::kThreads, coop::kSearchSmem, s>>>(rgba, w, h, bw, p, out, bc3, aligned, d.q, d.fq);
     });
 }
+
+int launch_batch_coop(const BatchItemDev *items, const TileDev *tiles, uint32_t *ctl, void *stream) {
+    static std::atomic<uint64_t> done{0};
+    const cudaError_t e = allow_smem(k_batch_coop, coop::kFitSmem, done);
+    if (e != cudaSuccess) return (int)e;
+    k_batch_coop<<<num_sms() * kCoopCtas, tpb::kThreads, coop::kFitSmem, (cudaStream_t)stream>>>(items, tiles, ctl);
+    return (int)cudaGetLastError();
+}
+
+int batch_coop_warps() { return num_sms() * kCoopCtas * coop::kWarps; }
 
 cudaError_t upload_coop_tables() { return cudaMemcpyToSymbol(g_tab, &host_tables(), sizeof(DevTables)); }
 

@@ -119,6 +119,11 @@ int launch_batch(const BatchItemDev *items, const TileDev *tiles, uint32_t *ctl,
 // runs the same tiles); grid <= 0 fills the SMs to the kernel's occupancy at that size
 int launch_batch(const BatchItemDev *items, const TileDev *tiles, uint32_t *ctl, int grid, int threads, void *stream);
 int batch_ctas_per_sm();
+// Whether a batch's BC1/BC3 encode with these settings goes to the cooperative kernel, and that kernel: it pulls
+// tiles[0 .. ctl[3]) through the counter ctl[2]. batch_coop_warps: its resident warps.
+bool coop_batch_setting(const qt_bc1_params &p);
+int launch_batch_coop(const BatchItemDev *items, const TileDev *tiles, uint32_t *ctl, void *stream);
+int batch_coop_warps();
 int batch_sms();
 
 }  // namespace qtk
