@@ -23,16 +23,15 @@
 //   - each output value = clamp((2^21 + sum(value * weight)) >> 22, 0, 255), 32-bit;
 //   - a horizontal pass over the source rows the vertical pass needs, to 8-bit
 //     values, then a vertical pass; a pass whose size does not change is skipped.
-// The weights are computed here on the host in double (x86-64, no FMA
-// contraction), exactly as Pillow does, and the device applies them.
+// The weights are computed on the device in double, operation by operation as Pillow does (-fmad=false: no
+// contraction): on the host they took 27-88 us of every call (470 us of a 2048^2 chain's 730), more than the resampling.
 
+#include <cooperative_groups.h>
 #include <cuda_runtime.h>
 
 #include <algorithm>
 #include <cmath>
 #include <cstdint>
-#include <cstring>
-#include <vector>
 
 #include "qt_internal.h"
 
@@ -40,51 +39,73 @@ namespace {
 
 constexpr int kPrecisionBits = 22;  // 32 - 8 - 2
 
-struct Taps {
-    int ksize = 0;
-    std::vector<int2> bounds;  // per output coordinate: first tap, tap count
-    std::vector<int32_t> kk;   // out * ksize fixed-point weights
-};
-
-double tri(double x) {
-    if (x < 0.0) x = -x;
-    return x < 1.0 ? 1.0 - x : 0.0;
-}
-
-Taps bilinear_taps(int in_size, int out_size) {
-    Taps t;
-    const float in0 = 0.0f, in1 = (float)in_size;
-    const double scale = (double)(in1 - in0) / out_size;
-    const double filterscale = scale < 1.0 ? 1.0 : scale;
-    const double support = 1.0 * filterscale;
-    t.ksize = (int)std::ceil(support) * 2 + 1;
-    t.bounds.resize((size_t)out_size);
-    t.kk.assign((size_t)out_size * t.ksize, 0);
-    std::vector<double> k((size_t)t.ksize);
-    for (int xx = 0; xx < out_size; xx++) {
-        const double center = in0 + (xx + 0.5) * scale;
-        double ww = 0.0;
-        const double ss = 1.0 / filterscale;
+// Size of one dimension's resampling: the widest output's tap count, and an output's first and one-past-last tap
+struct Scale {
+    int in_size, out_size, ksize;
+    double scale, support;
+    Scale(int in, int out) : in_size(in), out_size(out) {
+        scale = (double)(float)in / out;
+        support = 1.0 * (scale < 1.0 ? 1.0 : scale);
+        ksize = (int)std::ceil(support) * 2 + 1;
+    }
+    __host__ __device__ int2 bounds(int xx, double &center) const {
+        center = 0.0 + (xx + 0.5) * scale;
         int xmin = (int)(center - support + 0.5);
         if (xmin < 0) xmin = 0;
         int xmax = (int)(center + support + 0.5);
         if (xmax > in_size) xmax = in_size;
-        xmax -= xmin;
-        for (int x = 0; x < xmax; x++) {
-            const double w = tri((x + xmin - center + 0.5) * ss);
-            k[(size_t)x] = w;
-            ww += w;
-        }
-        for (int x = 0; x < xmax; x++)
-            if (ww != 0.0) k[(size_t)x] /= ww;
-        int32_t *row = t.kk.data() + (size_t)xx * t.ksize;
-        for (int x = 0; x < xmax; x++) {
-            const double v = k[(size_t)x];
-            row[x] = v < 0 ? (int32_t)(-0.5 + v * (1 << kPrecisionBits)) : (int32_t)(0.5 + v * (1 << kPrecisionBits));
-        }
-        t.bounds[(size_t)xx] = make_int2(xmin, xmax);
+        return make_int2(xmin, xmax);
     }
-    return t;
+};
+
+__device__ __forceinline__ double tri(double x) {
+    if (x < 0.0) x = -x;
+    return x < 1.0 ? 1.0 - x : 0.0;
+}
+
+// One output's fixed-point weights by a warp, into row[0 .. taps); returns its first tap and tap count. The weights' sum
+// runs in tap order, as Pillow's does, except for power-of-two scales (the halving chains of power-of-two
+// textures): there every weight is a multiple of 1 / (2 scale), so the sum is exact in any order and is a tree.
+__device__ __forceinline__ int2 output_taps(const Scale &S, int o, int32_t *row) {
+    const int lane = threadIdx.x & 31;
+    double center;
+    const int2 b = S.bounds(o, center);
+    const int xmin = b.x, n = b.y - b.x;
+    const double ss = 1.0 / S.support;
+    const bool pow2 = S.scale >= 1.0 && (__double_as_longlong(S.scale) & 0xFFFFFFFFFFFFFll) == 0;
+    double ww = 0.0;
+    if (pow2) {
+        for (int x = lane; x < n; x += 32) ww += tri((x + xmin - center + 0.5) * ss);
+#pragma unroll
+        for (int d = 16; d > 0; d >>= 1) ww += __shfl_xor_sync(0xffffffffu, ww, d);
+    } else {
+        for (int x0 = 0; x0 < n; x0 += 32) {
+            const int x = x0 + lane;
+            const double w = x < n ? tri((x + xmin - center + 0.5) * ss) : 0.0;
+#pragma unroll
+            for (int i = 0; i < 32; i++) ww += __shfl_sync(0xffffffffu, w, i);  // past the last tap: + 0.0
+        }
+    }
+#pragma unroll 4
+    for (int x = lane; x < n; x += 32) {
+        double k = tri((x + xmin - center + 0.5) * ss);
+        if (ww != 0.0) k /= ww;
+        row[x] = k < 0 ? (int32_t)(-0.5 + k * (1 << kPrecisionBits)) : (int32_t)(0.5 + k * (1 << kPrecisionBits));
+    }
+    return make_int2(xmin, n);
+}
+
+// The tap tables of both dimensions, one warp per output coordinate: per output its first tap and tap count, and ksize
+// weights
+__global__ void __launch_bounds__(256) k_taps(Scale h, Scale v, int2 *__restrict__ bounds_h, int32_t *__restrict__ kk_h,
+                                              int2 *__restrict__ bounds_v, int32_t *__restrict__ kk_v, int y_first) {
+    const long o = ((long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    if (o >= (long)h.out_size + v.out_size) return;
+    const bool vertical = o >= h.out_size;
+    const int i = (int)(vertical ? o - h.out_size : o);
+    const int2 b = vertical ? output_taps(v, i, kk_v + (size_t)i * v.ksize) : output_taps(h, i, kk_h + (size_t)i * h.ksize);
+    // the vertical pass reads the horizontal pass's rows, the first of them y_first
+    if ((threadIdx.x & 31) == 0) (vertical ? bounds_v : bounds_h)[i] = make_int2(vertical ? b.x - y_first : b.x, b.y);
 }
 
 __device__ __forceinline__ uint32_t clip8(int v) {
@@ -96,152 +117,271 @@ __device__ __forceinline__ uint32_t weighted(int s0, int s1, int s2, int s3) {
     return clip8(s0) | (clip8(s1) << 8) | (clip8(s2) << 16) | (clip8(s3) << 24);
 }
 
-// rows [y0, y0 + gridDim.y * k) of src (width w) -> dst rows [0, ...) of width dw
+__device__ __forceinline__ void add_tap(int s[4], uint32_t p, int c) {
+    s[0] += (int)(p & 0xFF) * c;
+    s[1] += (int)((p >> 8) & 0xFF) * c;
+    s[2] += (int)((p >> 16) & 0xFF) * c;
+    s[3] += (int)(p >> 24) * c;
+}
+
+// Horizontal pass: rows [y0, y0 + rows) of src (width w) -> rows [0, rows) of dst (width dw). G lanes share an output's
+// taps, G half the scale's power of two, so that neighbouring lanes read neighbouring texels at deep levels (one
+// output per lane strides by the scale); each lane sums them for four rows at once, which keeps four loads in flight
+// and reads each weight once. The 4 x 4 sums are exact integers; they meet by exchanging halves, so that lane bits
+// 0 and 1 end up with one row each and bits 2 and 3 with one channel each. Work is (row quad, output) pairs in
+// one sequence, so few outputs leave no lanes idle. A call from 2048^2 to 1024^2 took 89 us, to 256^2 108, to 32^2 38;
+// with this and the taps on the device 27, 24 and 22.
+template <int G>
 __global__ void __launch_bounds__(256) k_resample_h(const uint32_t *__restrict__ src, int w, int y0, int rows,
                                                     uint32_t *__restrict__ dst, int dw, const int2 *__restrict__ bounds,
                                                     const int32_t *__restrict__ kk, int ksize) {
-    const int x = blockIdx.x * blockDim.x + threadIdx.x;
-    if (x >= dw) return;
-    const int2 b = bounds[x];
-    const int32_t *k = kk + (size_t)x * ksize;
-    for (int y = blockIdx.y; y < rows; y += gridDim.y) {
-        const uint32_t *row = src + (size_t)(y0 + y) * w + b.x;
-        int s0 = 1 << (kPrecisionBits - 1), s1 = s0, s2 = s0, s3 = s0;
-        for (int t = 0; t < b.y; t++) {
-            const uint32_t p = __ldg(row + t);
+    const int sub = threadIdx.x & (G - 1);
+    const long quads = (rows + 3) / 4, groups = quads * dw, stride = (long)gridDim.x * (256 / G);
+    // a warp's lanes stay together: every lane of it runs the same number of iterations
+    for (long g0 = ((long)blockIdx.x * 256 + (threadIdx.x & ~31)) / G; g0 < groups; g0 += stride) {
+        const long go = g0 + (threadIdx.x & 31) / G;
+        const bool have = go < groups;
+        const long g = have ? go : groups - 1;  // lanes past the end take part in the exchanges
+        const int x = (int)(g % dw), y = 4 * (int)(g / dw);
+        const int2 b = bounds[x];
+        const int32_t *k = kk + (size_t)x * ksize;
+        const uint32_t *row[4];
+#pragma unroll
+        for (int r = 0; r < 4; r++) row[r] = src + (size_t)(y0 + (y + r < rows ? y + r : rows - 1)) * w + b.x;
+        int s[4][4] = {};
+#pragma unroll 4
+        for (int t = sub; t < b.y; t += G) {
             const int c = __ldg(k + t);
-            s0 += (int)(p & 0xFF) * c;
-            s1 += (int)((p >> 8) & 0xFF) * c;
-            s2 += (int)((p >> 16) & 0xFF) * c;
-            s3 += (int)(p >> 24) * c;
+#pragma unroll
+            for (int r = 0; r < 4; r++) add_tap(s[r], __ldg(row[r] + t), c);
         }
-        dst[(size_t)y * dw + x] = weighted(s0, s1, s2, s3);
+        int v[16];
+#pragma unroll
+        for (int i = 0; i < 16; i++) v[i] = s[i >> 2][i & 3];
+        int n = 16;
+#pragma unroll
+        for (int bit = 1; bit < G && bit < 16; bit <<= 1) {
+            n >>= 1;
+            const bool hi = sub & bit;
+#pragma unroll
+            for (int j = 0; j < 8; j++)
+                if (j < n) {
+                    const int send = hi ? v[j] : v[j + n], keep = hi ? v[j + n] : v[j];
+                    v[j] = keep + __shfl_xor_sync(0xffffffffu, send, bit);
+                }
+        }
+        if (G == 32) v[0] += __shfl_xor_sync(0xffffffffu, v[0], 16);
+        constexpr int kRows = G >= 4 ? 1 : 4 / G, kChannels = G >= 16 ? 1 : G >= 8 ? 2 : 4;
+        const int r0 = (G >= 2 ? (sub & 1) * 2 : 0) + (G >= 4 ? (sub >> 1) & 1 : 0);
+        const int c0 = (G >= 8 ? ((sub >> 2) & 1) * 2 : 0) + (G >= 16 ? (sub >> 3) & 1 : 0);
+#pragma unroll
+        for (int r = 0; r < kRows; r++) {
+            uint32_t p = 0;
+#pragma unroll
+            for (int c = 0; c < kChannels; c++) p |= clip8(v[r * kChannels + c] + (1 << (kPrecisionBits - 1))) << (8 * (c0 + c));
+            if (G >= 8) p |= __shfl_xor_sync(0xffffffffu, p, 4);
+            if (G >= 16) p |= __shfl_xor_sync(0xffffffffu, p, 8);
+            if (have && (sub >> 2) == 0 && y + r0 + r < rows) dst[(size_t)(y + r0 + r) * dw + x] = p;
+        }
     }
 }
 
-// src (width w, rows indexed by the shifted bounds) -> dst (w x dh)
+// Vertical pass: src (width w, rows indexed by the bounds) -> dst (w x dh). A CTA takes TX columns of one output row and
+// splits the taps over its 256 / TX groups of threads, whose sums meet in shared memory: few columns with
+// thousands of taps each (the deep levels) have as many threads to themselves as many columns with a few.
+template <int TX>
 __global__ void __launch_bounds__(256) k_resample_v(const uint32_t *__restrict__ src, int w, uint32_t *__restrict__ dst,
                                                     int dh, const int2 *__restrict__ bounds,
                                                     const int32_t *__restrict__ kk, int ksize) {
-    const int x = blockIdx.x * blockDim.x + threadIdx.x;
-    if (x >= w) return;
+    constexpr int TY = 256 / TX;
+    __shared__ int4 part[TY > 1 ? 256 : 1];
+    const int tx = threadIdx.x % TX, ty = threadIdx.x / TX, xo = blockIdx.x * TX + tx, x = xo < w ? xo : w - 1;
     for (int yy = blockIdx.y; yy < dh; yy += gridDim.y) {
         const int2 b = bounds[yy];
         const int32_t *k = kk + (size_t)yy * ksize;
-        int s0 = 1 << (kPrecisionBits - 1), s1 = s0, s2 = s0, s3 = s0;
-        for (int t = 0; t < b.y; t++) {
-            const uint32_t p = __ldg(src + (size_t)(b.x + t) * w + x);
-            const int c = __ldg(k + t);
-            s0 += (int)(p & 0xFF) * c;
-            s1 += (int)((p >> 8) & 0xFF) * c;
-            s2 += (int)((p >> 16) & 0xFF) * c;
-            s3 += (int)(p >> 24) * c;
-        }
-        dst[(size_t)yy * w + x] = weighted(s0, s1, s2, s3);
-    }
-}
-
-// Wide filters (the deep levels of a chain resize the original by up to its full
-// size, so one output sums thousands of taps): the taps of one output are split
-// over several threads and their partial sums added. The sums are exact 32-bit
-// integers, so the order of the additions does not change the result.
-
-// horizontal: one warp per output pixel, lanes stride over the taps (coalesced row reads)
-__global__ void __launch_bounds__(256) k_resample_h_wide(const uint32_t *__restrict__ src, int w, int y0, int rows,
-                                                         uint32_t *__restrict__ dst, int dw,
-                                                         const int2 *__restrict__ bounds,
-                                                         const int32_t *__restrict__ kk, int ksize) {
-    const int lane = threadIdx.x & 31;
-    const long nout = (long)dw * rows;
-    for (long o = ((long)blockIdx.x * blockDim.x + threadIdx.x) >> 5; o < nout; o += ((long)gridDim.x * blockDim.x) >> 5) {
-        const int y = (int)(o / dw), x = (int)(o - (long)y * dw);
-        const int2 b = bounds[x];
-        const int32_t *k = kk + (size_t)x * ksize;
-        const uint32_t *row = src + (size_t)(y0 + y) * w + b.x;
-        int s0 = 0, s1 = 0, s2 = 0, s3 = 0;
-        for (int t = lane; t < b.y; t += 32) {
-            const uint32_t p = __ldg(row + t);
-            const int c = __ldg(k + t);
-            s0 += (int)(p & 0xFF) * c;
-            s1 += (int)((p >> 8) & 0xFF) * c;
-            s2 += (int)((p >> 16) & 0xFF) * c;
-            s3 += (int)(p >> 24) * c;
-        }
+        int s[4] = {};
+#pragma unroll 4
+        for (int t = ty; t < b.y; t += TY) add_tap(s, __ldg(src + (size_t)(b.x + t) * w + x), __ldg(k + t));
+        if (TY > 1) {
+            part[threadIdx.x] = make_int4(s[0], s[1], s[2], s[3]);
+            __syncthreads();
 #pragma unroll
-        for (int d = 16; d > 0; d >>= 1) {
-            s0 += __shfl_xor_sync(0xffffffffu, s0, d);
-            s1 += __shfl_xor_sync(0xffffffffu, s1, d);
-            s2 += __shfl_xor_sync(0xffffffffu, s2, d);
-            s3 += __shfl_xor_sync(0xffffffffu, s3, d);
+            for (int d = 128; d >= TX; d >>= 1) {
+                if (threadIdx.x < d) {
+                    const int4 o = part[threadIdx.x + d];
+                    int4 &a = part[threadIdx.x];
+                    a = make_int4(a.x + o.x, a.y + o.y, a.z + o.z, a.w + o.w);
+                }
+                __syncthreads();
+            }
+            const int4 a = part[tx];
+            s[0] = a.x; s[1] = a.y; s[2] = a.z; s[3] = a.w;
+            __syncthreads();  // the next row's sums overwrite part
         }
-        if (lane == 0) {
-            const int half = 1 << (kPrecisionBits - 1);
-            dst[(size_t)y * dw + x] = weighted(s0 + half, s1 + half, s2 + half, s3 + half);
-        }
+        const int half = 1 << (kPrecisionBits - 1);
+        if (ty == 0 && xo < w) dst[(size_t)yy * w + x] = weighted(s[0] + half, s[1] + half, s[2] + half, s[3] + half);
     }
 }
 
-// vertical: a CTA of 32 columns x 8 tap groups; the 8 partial sums of a column meet in shared memory
-__global__ void __launch_bounds__(256) k_resample_v_wide(const uint32_t *__restrict__ src, int w,
-                                                         uint32_t *__restrict__ dst, int dh,
-                                                         const int2 *__restrict__ bounds,
-                                                         const int32_t *__restrict__ kk, int ksize) {
-    __shared__ int4 part[8][32];
-    const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
-    const int x = blockIdx.x * 32 + tx;
-    for (int yy = blockIdx.y; yy < dh; yy += gridDim.y) {
-        const int2 b = bounds[yy];
-        const int32_t *k = kk + (size_t)yy * ksize;
-        int s0 = 0, s1 = 0, s2 = 0, s3 = 0;
-        if (x < w)
-            for (int t = ty; t < b.y; t += 8) {
-                const uint32_t p = __ldg(src + (size_t)(b.x + t) * w + x);
-                const int c = __ldg(k + t);
-                s0 += (int)(p & 0xFF) * c;
-                s1 += (int)((p >> 8) & 0xFF) * c;
-                s2 += (int)((p >> 16) & 0xFF) * c;
-                s3 += (int)(p >> 24) * c;
-            }
-        part[ty][tx] = make_int4(s0, s1, s2, s3);
-        __syncthreads();
-        if (ty == 0 && x < w) {
-            const int half = 1 << (kPrecisionBits - 1);
+// One output's weights by one thread (few taps)
+__device__ __forceinline__ int2 output_taps_thread(const Scale &S, int o, int32_t *row) {
+    double center;
+    const int2 b = S.bounds(o, center);
+    const int xmin = b.x, n = b.y - b.x;
+    const double ss = 1.0 / S.support;
+    double ww = 0.0;
+    for (int x = 0; x < n; x++) ww += tri((x + xmin - center + 0.5) * ss);
+    for (int x = 0; x < n; x++) {
+        double k = tri((x + xmin - center + 0.5) * ss);
+        if (ww != 0.0) k /= ww;
+        row[x] = k < 0 ? (int32_t)(-0.5 + k * (1 << kPrecisionBits)) : (int32_t)(0.5 + k * (1 << kPrecisionBits));
+    }
+    return make_int2(xmin, n);
+}
+
+// Both passes of a small texture in one kernel: a cluster of 8 CTAs per output row, which splits the source rows that it
+// needs. Each CTA computes the taps (few: a thread per output, many: a warp), the horizontal pass of its rows and
+// their share of the vertical sums, all in shared memory; the CTAs then add the shares, each for some of the columns. A
+// row of the horizontal pass is computed by the ~2 output rows that need it; for that the call is one launch without
+// scratch memory: three launches and the allocation take 22 us of host time, one 11, and a chain's small levels have
+// nothing else. G as in k_resample_h.
+constexpr int kSplit = 8;
+struct SmallLayout {  // word offsets in shared memory
+    int kk_v, bounds_h, kk_h, rows, share, words;
+    SmallLayout(const Scale &h, const Scale &v) {
+        const int nv = v.in_size == v.out_size ? 1 : std::min(v.ksize, v.in_size);
+        kk_v = 0;
+        bounds_h = (v.ksize + 1) / 2 * 2;
+        kk_h = bounds_h + 2 * h.out_size;
+        rows = kk_h + h.out_size * h.ksize;
+        share = (rows + (nv + kSplit - 1) / kSplit * h.out_size + 3) / 4 * 4;
+        words = share + 4 * h.out_size;
+    }
+};
+
+template <int G>
+__global__ void __cluster_dims__(kSplit, 1, 1) __launch_bounds__(256) k_resize_small(const uint32_t *__restrict__ src, Scale h, Scale v, uint32_t *__restrict__ dst, SmallLayout L) {
+    extern __shared__ __align__(16) int32_t sm[];  // share is read as int4
+    __shared__ int2 bv;
+    const cooperative_groups::cluster_group cluster = cooperative_groups::this_cluster();
+    int2 *const bounds_h = reinterpret_cast<int2 *>(sm + L.bounds_h);
+    uint32_t *const mid = reinterpret_cast<uint32_t *>(sm + L.rows);
+    int4 *const share = reinterpret_cast<int4 *>(sm + L.share);
+    const int rank = (int)cluster.block_rank(), yy = blockIdx.x / kSplit;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, w = h.in_size, dw = h.out_size;
+    const bool need_h = w != dw, need_v = v.in_size != v.out_size;
+    const int half = 1 << (kPrecisionBits - 1);
+    if (warp == 7) {
+        const int2 b = need_v ? output_taps(v, yy, sm + L.kk_v) : make_int2(yy, 1);
+        if (lane == 0) bv = b;
+    }
+    if (need_h && h.ksize <= 32) {
+        for (int x = threadIdx.x; x < dw; x += 256) bounds_h[x] = output_taps_thread(h, x, sm + L.kk_h + x * h.ksize);
+    } else if (need_h) {
+        for (int x = warp; x < dw; x += 8) {
+            const int2 b = output_taps(h, x, sm + L.kk_h + x * h.ksize);
+            if (lane == 0) bounds_h[x] = b;
+        }
+    }
+    __syncthreads();
+    // horizontal: source rows bv.x + rank, + 8, ... -> mid, G lanes an output
+    const int rows = bv.y > rank ? (bv.y - rank + kSplit - 1) / kSplit : 0, items = rows * dw, sub = lane & (G - 1);
+    for (int i0 = (threadIdx.x & ~31) / G; i0 < items; i0 += 256 / G) {
+        const int io = i0 + lane / G, i = io < items ? io : items - 1;
+        const int r = i / dw, x = i - r * dw;
+        const uint32_t *row = src + (size_t)(bv.x + rank + r * kSplit) * w;
+        uint32_t p;
+        if (need_h) {
+            const int2 b = bounds_h[x];
+            const int32_t *k = sm + L.kk_h + x * h.ksize;
+            int s[4] = {};
+#pragma unroll 4
+            for (int t = sub; t < b.y; t += G) add_tap(s, __ldg(row + b.x + t), k[t]);
+#pragma unroll
+            for (int d = 1; d < G; d <<= 1)
+#pragma unroll
+                for (int c = 0; c < 4; c++) s[c] += __shfl_xor_sync(0xffffffffu, s[c], d);
+            p = weighted(s[0] + half, s[1] + half, s[2] + half, s[3] + half);
+        } else {
+            p = __ldg(row + x);
+        }
+        if (io < items && sub == 0) mid[io] = p;
+    }
+    __syncthreads();
+    // vertical: this CTA's rows' share of every column's sums, then the columns' sums over the CTAs
+    if (need_v)
+        for (int x = threadIdx.x; x < dw; x += 256) {
+            int s[4] = {};
+            for (int r = 0; r < rows; r++) add_tap(s, mid[r * dw + x], sm[L.kk_v + rank + r * kSplit]);
+            share[x] = make_int4(s[0], s[1], s[2], s[3]);
+        }
+    cluster.sync();
+    for (int x = rank + kSplit * threadIdx.x; x < dw; x += kSplit * 256) {
+        uint32_t p;
+        if (need_v) {
             int4 a = make_int4(half, half, half, half);
 #pragma unroll
-            for (int g = 0; g < 8; g++) {
-                a.x += part[g][tx].x;
-                a.y += part[g][tx].y;
-                a.z += part[g][tx].z;
-                a.w += part[g][tx].w;
+            for (int c = 0; c < kSplit; c++) {
+                const int4 o = cluster.map_shared_rank(share, c)[x];
+                a = make_int4(a.x + o.x, a.y + o.y, a.z + o.z, a.w + o.w);
             }
-            dst[(size_t)yy * w + x] = weighted(a.x, a.y, a.z, a.w);
+            p = weighted(a.x, a.y, a.z, a.w);
+        } else {
+            p = cluster.map_shared_rank(mid, 0)[x];  // the one row is rank 0's
         }
-        __syncthreads();
+        dst[(size_t)yy * dw + x] = p;
     }
+    cluster.sync();  // the others' reads of this CTA's shared memory
 }
 
-constexpr int kWideTaps = 16;  // above this many taps per output, the split kernels run
+// up to this many source texels
+constexpr long kSmallTexels = 512L * 512;
 
-dim3 grid_2d(int x, int y) { return dim3((unsigned)((x + 255) / 256), (unsigned)(y < 65535 ? y : 65535)); }
+bool small_resize(const Scale &h, const Scale &v) {
+    return (long)h.in_size * v.in_size <= kSmallTexels && (long)SmallLayout(h, v).words * 4 <= 46 * 1024;
+}
+
+template <int G> void resize_small_g(const uint32_t *in, const Scale &h, const Scale &v, uint32_t *out, cudaStream_t s) {
+    const SmallLayout L(h, v);
+    k_resize_small<G><<<(unsigned)v.out_size * kSplit, 256, (size_t)L.words * 4, s>>>(in, h, v, out, L);
+}
+
+void resize_small(const uint32_t *in, const Scale &h, const Scale &v, uint32_t *out, cudaStream_t s) {
+    const int scale = h.in_size / h.out_size / 2;
+    if (scale >= 32) resize_small_g<32>(in, h, v, out, s);
+    else if (scale >= 8) resize_small_g<8>(in, h, v, out, s);
+    else if (scale >= 2) resize_small_g<2>(in, h, v, out, s);
+    else resize_small_g<1>(in, h, v, out, s);
+}
+
+template <int G>
+void resample_h_g(const uint32_t *in, int w, int y0, int rows, uint32_t *out, int dw, const int2 *b, const int32_t *k, int ksize, cudaStream_t s) {
+    const long ctas = std::min<long>(((long)dw * ((rows + 3) / 4) * G + 255) / 256, 148L * 64);
+    k_resample_h<G><<<(unsigned)ctas, 256, 0, s>>>(in, w, y0, rows, out, dw, b, k, ksize);
+}
 
 void resample_h(const uint32_t *in, int w, int y0, int rows, uint32_t *out, int dw, const int2 *b, const int32_t *k,
                 int ksize, cudaStream_t s) {
-    if (ksize > kWideTaps) {
-        const long warps = (long)dw * rows;
-        const long ctas = std::min<long>((warps + 7) / 8, 148L * 64);
-        k_resample_h_wide<<<(unsigned)ctas, 256, 0, s>>>(in, w, y0, rows, out, dw, b, k, ksize);
-    } else {
-        k_resample_h<<<grid_2d(dw, rows), 256, 0, s>>>(in, w, y0, rows, out, dw, b, k, ksize);
-    }
+    const int scale = w / dw / 2;  // lanes per output: half the scale's power of two
+    if (scale >= 32) resample_h_g<32>(in, w, y0, rows, out, dw, b, k, ksize, s);
+    else if (scale >= 16) resample_h_g<16>(in, w, y0, rows, out, dw, b, k, ksize, s);
+    else if (scale >= 8) resample_h_g<8>(in, w, y0, rows, out, dw, b, k, ksize, s);
+    else if (scale >= 4) resample_h_g<4>(in, w, y0, rows, out, dw, b, k, ksize, s);
+    else if (scale >= 2) resample_h_g<2>(in, w, y0, rows, out, dw, b, k, ksize, s);
+    else resample_h_g<1>(in, w, y0, rows, out, dw, b, k, ksize, s);
+}
+
+template <int TX>
+void resample_v_x(const uint32_t *in, int w, uint32_t *out, int dh, const int2 *b, const int32_t *k, int ksize, cudaStream_t s) {
+    k_resample_v<TX><<<dim3((unsigned)((w + TX - 1) / TX), (unsigned)std::min(dh, 65535)), 256, 0, s>>>(in, w, out, dh, b, k, ksize);
 }
 
 void resample_v(const uint32_t *in, int w, uint32_t *out, int dh, const int2 *b, const int32_t *k, int ksize,
                 cudaStream_t s) {
-    if (ksize > kWideTaps)
-        k_resample_v_wide<<<dim3((unsigned)((w + 31) / 32), (unsigned)(dh < 65535 ? dh : 65535)), 256, 0, s>>>(
-            in, w, out, dh, b, k, ksize);
-    else
-        k_resample_v<<<grid_2d(w, dh), 256, 0, s>>>(in, w, out, dh, b, k, ksize);
+    if (ksize <= 16) resample_v_x<256>(in, w, out, dh, b, k, ksize, s);
+    else if (ksize <= 128) resample_v_x<32>(in, w, out, dh, b, k, ksize, s);
+    else if (w >= 64 || (w >= 8 && ksize <= 1024)) resample_v_x<8>(in, w, out, dh, b, k, ksize, s);
+    else resample_v_x<1>(in, w, out, dh, b, k, ksize, s);
 }
 
 }  // namespace
@@ -259,30 +399,28 @@ extern "C" int qt_resize_bilinear_device(const uint8_t *src, int w, int h, uint8
         return e == cudaSuccess ? QT_OK : qtk::cuda_error((int)e, "resize copy");
     }
     const bool need_h = dw != w, need_v = dh != h;
-    const Taps th = bilinear_taps(w, dw);
-    Taps tv = bilinear_taps(h, dh);
-    const int y_first = tv.bounds[0].x, y_last = tv.bounds[(size_t)dh - 1].x + tv.bounds[(size_t)dh - 1].y;
-    if (need_h)
-        for (int2 &b : tv.bounds) b.x -= y_first;  // the vertical pass reads the horizontal pass's rows
+    const Scale sh(w, dw), sv(h, dh);
+    if (small_resize(sh, sv)) {
+        resize_small(reinterpret_cast<const uint32_t *>(src), sh, sv, reinterpret_cast<uint32_t *>(dst), s);
+        e = cudaGetLastError();
+        return e == cudaSuccess ? QT_OK : qtk::cuda_error((int)e, "resize");
+    }
+    double centre;
+    const int y_first = sv.bounds(0, centre).x, tmp_rows = sv.bounds(dh - 1, centre).y - y_first;
 
-    // one buffer for both tap tables (stream-ordered, freed after the passes); every table
-    // starts on a 16-byte boundary (the bounds are read as 8-byte int2)
+    // one stream-ordered block for both tap tables and the horizontal pass's rows; every part starts on a 16-byte
+    // boundary (the bounds are read as 8-byte int2)
     const auto al = [](size_t n) { return (n + 15) / 16 * 16; };
-    const size_t bh = th.bounds.size() * sizeof(int2), kh = th.kk.size() * sizeof(int32_t);
-    const size_t bv = tv.bounds.size() * sizeof(int2), kv = tv.kk.size() * sizeof(int32_t);
-    const size_t o_kh = al(bh), o_bv = al(o_kh + kh), o_kv = al(o_bv + bv);
-    std::vector<uint8_t> host(o_kv + kv);
-    std::memcpy(host.data(), th.bounds.data(), bh);
-    std::memcpy(host.data() + o_kh, th.kk.data(), kh);
-    std::memcpy(host.data() + o_bv, tv.bounds.data(), bv);
-    std::memcpy(host.data() + o_kv, tv.kk.data(), kv);
+    const size_t o_kh = al((size_t)dw * sizeof(int2)), o_bv = o_kh + al((size_t)dw * sh.ksize * sizeof(int32_t));
+    const size_t o_kv = o_bv + al((size_t)dh * sizeof(int2)), o_tmp = o_kv + al((size_t)dh * sv.ksize * sizeof(int32_t));
     uint8_t *d_taps = nullptr;
-    uint32_t *d_tmp = nullptr;
-    const int tmp_rows = y_last - y_first;
-    if ((e = qtk::scratch_alloc((void **)&d_taps, host.size(), s)) != cudaSuccess) return qtk::cuda_error((int)e, "resize taps");
-    // from pageable memory: the call returns once `host` has been staged
-    e = cudaMemcpyAsync(d_taps, host.data(), host.size(), cudaMemcpyHostToDevice, s);
-    if (e == cudaSuccess && need_h && need_v) e = qtk::scratch_alloc((void **)&d_tmp, (size_t)dw * tmp_rows * 4, s);
+    if ((e = qtk::scratch_alloc((void **)&d_taps, o_tmp + (need_h && need_v ? (size_t)dw * tmp_rows * 4 : 0), s)) != cudaSuccess)
+        return qtk::cuda_error((int)e, "resize scratch");
+    uint32_t *const d_tmp = reinterpret_cast<uint32_t *>(d_taps + o_tmp);
+    k_taps<<<(unsigned)(((long)dw + dh + 7) / 8), 256, 0, s>>>(sh, sv, reinterpret_cast<int2 *>(d_taps), reinterpret_cast<int32_t *>(d_taps + o_kh),
+                                                              reinterpret_cast<int2 *>(d_taps + o_bv), reinterpret_cast<int32_t *>(d_taps + o_kv),
+                                                              need_h ? y_first : 0);
+    e = cudaGetLastError();
     if (e == cudaSuccess) {
         const int2 *b_h = reinterpret_cast<const int2 *>(d_taps);
         const int32_t *k_h = reinterpret_cast<const int32_t *>(d_taps + o_kh);
@@ -291,16 +429,15 @@ extern "C" int qt_resize_bilinear_device(const uint8_t *src, int w, int h, uint8
         const uint32_t *in = reinterpret_cast<const uint32_t *>(src);
         uint32_t *out = reinterpret_cast<uint32_t *>(dst);
         if (need_h && need_v) {
-            resample_h(in, w, y_first, tmp_rows, d_tmp, dw, b_h, k_h, th.ksize, s);
-            resample_v(d_tmp, dw, out, dh, b_v, k_v, tv.ksize, s);
+            resample_h(in, w, y_first, tmp_rows, d_tmp, dw, b_h, k_h, sh.ksize, s);
+            resample_v(d_tmp, dw, out, dh, b_v, k_v, sv.ksize, s);
         } else if (need_h) {
-            resample_h(in, w, 0, h, out, dw, b_h, k_h, th.ksize, s);
+            resample_h(in, w, 0, h, out, dw, b_h, k_h, sh.ksize, s);
         } else {
-            resample_v(in, w, out, dh, b_v, k_v, tv.ksize, s);
+            resample_v(in, w, out, dh, b_v, k_v, sv.ksize, s);
         }
         e = cudaGetLastError();
     }
-    qtk::scratch_free(d_tmp, s);
     qtk::scratch_free(d_taps, s);
     return e == cudaSuccess ? QT_OK : qtk::cuda_error((int)e, "resize");
 }
