@@ -2,19 +2,20 @@
 // include/quicktex_cuda.h).
 //
 // A qt_batch owns, per device: the device work queue (texture descriptors,
-// tiles, and a four-word control block: head and end of each of two tile
-// ranges), pinned host staging for it, and a CUDA graph holding the persistent
-// launch. Every qt_batch_run cuts the textures into tiles (tile size per
+// tiles, and a control block: head and end of each kernel's range of tiles),
+// pinned host staging for it, and a CUDA graph holding the persistent launch. Every qt_batch_run cuts the textures into tiles (tile size per
 // format/level from the tuning rules), orders the tiles by estimated cost,
 // heaviest first (so the long tiles start early and the cheap ones fill the
-// tail), uploads the queue, and replays the graph. The tiles of textures whose
-// cluster fit runs cooperatively (qt_bc1_coop.cuh: levels 16-19) go to a
-// kernel of their own beside k_batch, in the same graph. Graphs are
-// re-captured only when a queue buffer has to grow.
+// tail), uploads the queue, and replays the graph. BC1/BC3 encodes go to kernels
+// of their own beside k_batch, in the same graph: the cooperative encoder
+// (levels 16-19) and encoders specialised by interpolator, error mode and
+// colour mode. A graph is built the first time a run holds that set of kernels,
+// and again when a queue buffer has to grow.
 
 #include <algorithm>
 #include <cstdlib>
 #include <cstring>
+#include <map>
 #include <mutex>
 #include <vector>
 
@@ -74,9 +75,7 @@ struct qt_batch {
     uint32_t *d_ctl = nullptr, *h_ctl = nullptr;
     cudaEvent_t staged = nullptr;     // the last upload from the pinned staging buffers
     cudaEvent_t done = nullptr;       // the last persistent launch (the queue is in use until then)
-    cudaStream_t capture[2] = {};     // private streams the graphs are captured on: the cooperative kernel's, k_batch's
-    cudaEvent_t fork = nullptr, join = nullptr;
-    cudaGraphExec_t exec[4] = {};     // by what a run holds: 1 tiles of k_batch, 2 of the cooperative kernel, 3 both
+    std::map<uint32_t, cudaGraphExec_t> exec;  // by the set of kernels (bit k: kind k) that a run holds tiles for
 
     qt_batch() {
         for (int op = 0; op < 2; op++)
@@ -100,12 +99,11 @@ namespace {
 
 // the queue's smallest capacity: a run's tiles are cut finer to fill the GPU only while they fit it
 constexpr size_t kMinTiles = 16384;
+constexpr size_t kCtlBytes = 2 * qtk::kBatchKinds * sizeof(uint32_t);
 
 void drop_graphs(qt_batch *b) {
-    for (cudaGraphExec_t &e : b->exec) {
-        if (e) cudaGraphExecDestroy(e);
-        e = nullptr;
-    }
+    for (auto &e : b->exec) cudaGraphExecDestroy(e.second);
+    b->exec.clear();
 }
 
 void free_buffers(qt_batch *b) {
@@ -140,31 +138,35 @@ int grow(qt_batch *b, size_t items, size_t tiles) {
     return QT_OK;
 }
 
-// Captures a run's launches once (replays read the queue through fixed pointers): k_batch (kind 1), the cooperative
-// kernel (2) or both side by side (3).
-int capture(qt_batch *b, int kind) {
-    const int grid = b->ctas_per_sm > 0 ? qtk::batch_sms() * b->ctas_per_sm : 0;
-    cudaError_t e = cudaStreamBeginCapture(b->capture[0], cudaStreamCaptureModeThreadLocal);
-    if (e != cudaSuccess) return qtk::cuda_error((int)e, "graph capture");
-    int lrc = 0;
-    if (kind == 3 && (e = cudaEventRecord(b->fork, b->capture[0])) == cudaSuccess) e = cudaStreamWaitEvent(b->capture[1], b->fork, 0);
-    if (e == cudaSuccess && (kind & 2)) lrc = qtk::launch_batch_coop(b->d_items, b->d_tiles, b->d_ctl, b->capture[0]);
-    if (e == cudaSuccess && !lrc && (kind & 1))
-        lrc = qtk::launch_batch(b->d_items, b->d_tiles, b->d_ctl, grid, b->threads, b->capture[kind == 3]);
-    if (e == cudaSuccess && kind == 3 && (e = cudaEventRecord(b->join, b->capture[1])) == cudaSuccess)
-        e = cudaStreamWaitEvent(b->capture[0], b->join, 0);
+// Builds the graph of a run's launches, side by side (replays read the queue through fixed pointers): the kernels of `kinds`
+int build_graph(qt_batch *b, uint32_t kinds) {
     cudaGraph_t g = nullptr;
-    const cudaError_t end = cudaStreamEndCapture(b->capture[0], &g);
-    if (lrc || e != cudaSuccess || end != cudaSuccess) {
-        if (g) cudaGraphDestroy(g);
-        return lrc ? qtk::cuda_error(lrc, "batch launch") : qtk::cuda_error((int)(e != cudaSuccess ? e : end), "graph capture");
+    cudaError_t e = cudaGraphCreate(&g, 0);
+    for (int k = 0; k < qtk::kBatchKinds && e == cudaSuccess; k++) {
+        if (!((kinds >> k) & 1u)) continue;
+        qtk::BatchLaunch l;
+        if ((e = (cudaError_t)qtk::batch_launch(k, b->ctas_per_sm, b->threads, &l)) != cudaSuccess) break;
+        uint32_t *ctl = b->d_ctl + 2 * k;
+        void *args[] = {&b->d_items, &b->d_tiles, &ctl};
+        cudaKernelNodeParams np = {};
+        np.func = const_cast<void *>(l.func);
+        np.gridDim = dim3((unsigned)l.grid);
+        np.blockDim = dim3((unsigned)l.threads);
+        np.sharedMemBytes = (unsigned)l.smem;
+        np.kernelParams = args;
+        cudaGraphNode_t node;
+        e = cudaGraphAddKernelNode(&node, g, nullptr, 0, &np);
+        if (e == cudaSuccess && k == 1) {  // its tiles are the long ones: they start first
+            cudaLaunchAttributeValue v = {};
+            v.priority = -1;
+            e = cudaGraphKernelNodeSetAttribute(node, cudaLaunchAttributePriority, &v);
+        }
     }
-    e = cudaGraphInstantiate(&b->exec[kind], g, 0);
-    cudaGraphDestroy(g);
-    if (e != cudaSuccess) {
-        b->exec[kind] = nullptr;
-        return qtk::cuda_error((int)e, "graph instantiate");
-    }
+    cudaGraphExec_t exec = nullptr;
+    if (e == cudaSuccess) e = cudaGraphInstantiate(&exec, g, 0);
+    if (g) cudaGraphDestroy(g);
+    if (e != cudaSuccess) return qtk::cuda_error((int)e, "building the batch's graph");
+    b->exec[kinds] = exec;
     return QT_OK;
 }
 
@@ -207,13 +209,8 @@ int qt_batch_create(int device, qt_batch **out) {
         b->device = device;
         if ((e = cudaEventCreateWithFlags(&b->staged, cudaEventDisableTiming)) != cudaSuccess ||
             (e = cudaEventCreateWithFlags(&b->done, cudaEventDisableTiming)) != cudaSuccess ||
-            (e = cudaEventCreateWithFlags(&b->fork, cudaEventDisableTiming)) != cudaSuccess ||
-            (e = cudaEventCreateWithFlags(&b->join, cudaEventDisableTiming)) != cudaSuccess ||
-            // the cooperative kernel's node carries its stream's priority: its tiles, the long ones, start first
-            (e = cudaStreamCreateWithPriority(&b->capture[0], cudaStreamNonBlocking, -1)) != cudaSuccess ||
-            (e = cudaStreamCreateWithPriority(&b->capture[1], cudaStreamNonBlocking, 0)) != cudaSuccess ||
-            (e = cudaMalloc(&b->d_ctl, 4 * sizeof(uint32_t))) != cudaSuccess ||
-            (e = cudaHostAlloc((void **)&b->h_ctl, 4 * sizeof(uint32_t), cudaHostAllocDefault)) != cudaSuccess) {
+            (e = cudaMalloc(&b->d_ctl, kCtlBytes)) != cudaSuccess ||
+            (e = cudaHostAlloc((void **)&b->h_ctl, kCtlBytes, cudaHostAllocDefault)) != cudaSuccess) {
             rc = qtk::cuda_error((int)e, "creating a batch");
             qt_batch_destroy(b);
             b = nullptr;
@@ -235,10 +232,6 @@ int qt_batch_destroy(qt_batch *b) {
     cudaFreeHost(b->h_ctl);
     if (b->staged) cudaEventDestroy(b->staged);
     if (b->done) cudaEventDestroy(b->done);
-    if (b->fork) cudaEventDestroy(b->fork);
-    if (b->join) cudaEventDestroy(b->join);
-    for (cudaStream_t s : b->capture)
-        if (s) cudaStreamDestroy(s);
     cudaSetDevice(prev);
     delete b;
     return QT_OK;
@@ -311,10 +304,10 @@ int qt_batch_run(qt_batch *b, const qt_batch_item *items, size_t n, void *stream
     std::vector<qtk::BatchItemDev> dev(n);
     struct Plan {
         Rule rule;
-        bool coop;
+        int kind;
     };
     std::vector<Plan> plan(n);
-    double work[2] = {0, 0};  // of k_batch, of the cooperative kernel
+    double work[2] = {0, 0};  // of the kernels that run a block per lane, of the cooperative one
     size_t coarse = 0;
     for (size_t i = 0; i < n; i++) {
         const qt_batch_item &it = items[i];
@@ -338,40 +331,38 @@ int qt_batch_run(qt_batch *b, const qt_batch_item *items, size_t n, void *stream
         const bool leveled = it.op == QT_OP_ENCODE && (it.format == 1 || it.format == 3);
         Plan &pl = plan[i];
         pl.rule = b->rules[rule_index(it.op, it.format, leveled ? qtk_level_of(it.params) : 0)];
-        pl.coop = leveled && qtk::coop_batch_setting(it.params);
-        work[pl.coop] += (double)pl.rule.cost * (double)nb;
+        pl.kind = qtk::batch_kind(it.op, it.format, it.params);
+        work[pl.kind == 1] += (double)pl.rule.cost * (double)nb;
         coarse += (size_t)((nb + pl.rule.tile_blocks - 1) / pl.rule.tile_blocks);
     }
-    // Tiles of the rules' sizes, or smaller where a kernel's resident warps would have fewer than four each (a short
-    // batch waits for its longest tile): a cooperative warp works on one block at a time, so its tiles may fall to a few
-    // blocks; k_batch's keep 32, a block per lane.
-    const double warps[2] = {(double)qtk::batch_sms() * 16, (double)qtk::batch_coop_warps()};
-    const size_t finer = 4 * (size_t)(warps[0] + warps[1]) + n;
+    // Tiles of the rules' sizes, or smaller where the resident warps would have fewer than four each (a short batch
+    // waits for its longest tile): a cooperative warp works on one block at a time, so its tiles may fall to a few
+    // blocks; the others keep 32, a block per lane.
+    const double warps = (double)qtk::batch_sms() * 16;
+    const size_t finer = 8 * (size_t)warps + n;
     const bool cut = coarse + finer <= std::max(b->cap_tiles, kMinTiles);
     struct Tile {
+        int kind;
         float cost;
         qtk::TileDev t;
     };
-    std::vector<Tile> tiles, rest;  // of the cooperative kernel, of k_batch; heaviest first
+    std::vector<Tile> tiles;
     for (size_t i = 0; i < n; i++) {
         const Plan &pl = plan[i];
+        const bool coop = pl.kind == 1;
         const uint64_t nb = (uint64_t)dev[i].bw * dev[i].bh;
         uint64_t tb = pl.rule.tile_blocks;
         if (cut) {
-            const uint64_t fill = (uint64_t)(work[pl.coop] / (warps[pl.coop] * 4) / pl.rule.cost) + 1;
-            tb = std::min(tb, pl.coop ? fill : (fill + 31) / 32 * 32);
+            const uint64_t fill = (uint64_t)(work[coop] / (warps * 4) / pl.rule.cost) + 1;
+            tb = std::min(tb, coop ? fill : (fill + 31) / 32 * 32);
         }
-        std::vector<Tile> &to = pl.coop ? tiles : rest;
         for (uint64_t s0 = 0; s0 < nb; s0 += tb) {
             const uint32_t cnt = (uint32_t)std::min<uint64_t>(tb, nb - s0);
-            to.push_back({pl.rule.cost * cnt, {(uint32_t)i, (uint32_t)s0, cnt, 0u}});
+            tiles.push_back({pl.kind, pl.rule.cost * cnt, {(uint32_t)i, (uint32_t)s0, cnt, 0u}});
         }
     }
-    const auto heavier = [](const Tile &a, const Tile &c) { return a.cost > c.cost; };
-    std::stable_sort(tiles.begin(), tiles.end(), heavier);
-    std::stable_sort(rest.begin(), rest.end(), heavier);
-    const size_t ncoop = tiles.size();
-    tiles.insert(tiles.end(), rest.begin(), rest.end());
+    // each kernel's tiles together, heaviest first
+    std::stable_sort(tiles.begin(), tiles.end(), [](const Tile &a, const Tile &c) { return a.kind != c.kind ? a.kind < c.kind : a.cost > c.cost; });
     b->last_tiles = tiles.size();
     if (tiles.size() > 0xFFFFFFFFull) return qtk::set_error(QT_ERR_ARG, "too many tiles");
     if (tiles.empty()) return QT_OK;
@@ -381,23 +372,25 @@ int qt_batch_run(qt_batch *b, const qt_batch_item *items, size_t n, void *stream
     if (e != cudaSuccess) return qtk::cuda_error((int)e, "batch staging");
     std::memcpy(b->h_items, dev.data(), n * sizeof(qtk::BatchItemDev));
     for (size_t i = 0; i < tiles.size(); i++) b->h_tiles[i] = tiles[i].t;
-    b->h_ctl[0] = (uint32_t)ncoop;  // k_batch's tiles follow the cooperative kernel's
-    b->h_ctl[1] = (uint32_t)tiles.size();
-    b->h_ctl[2] = 0;
-    b->h_ctl[3] = (uint32_t)ncoop;
+    uint32_t kinds = 0;
+    for (size_t i = 0; i < tiles.size(); i++) {
+        const int k = tiles[i].kind;
+        if (!((kinds >> k) & 1u)) b->h_ctl[2 * k] = (uint32_t)i;
+        b->h_ctl[2 * k + 1] = (uint32_t)i + 1;
+        kinds |= 1u << k;
+    }
     cudaStream_t s = (cudaStream_t)stream;
     // runs on other streams: do not overwrite the queue before the previous launch finished reading it
     if ((e = cudaStreamWaitEvent(s, b->done, 0)) != cudaSuccess) return qtk::cuda_error((int)e, "batch ordering");
     if ((e = cudaMemcpyAsync(b->d_items, b->h_items, n * sizeof(qtk::BatchItemDev), cudaMemcpyHostToDevice, s)) != cudaSuccess ||
         (e = cudaMemcpyAsync(b->d_tiles, b->h_tiles, tiles.size() * sizeof(qtk::TileDev), cudaMemcpyHostToDevice, s)) != cudaSuccess ||
-        (e = cudaMemcpyAsync(b->d_ctl, b->h_ctl, 4 * sizeof(uint32_t), cudaMemcpyHostToDevice, s)) != cudaSuccess ||
+        (e = cudaMemcpyAsync(b->d_ctl, b->h_ctl, kCtlBytes, cudaMemcpyHostToDevice, s)) != cudaSuccess ||
         (e = cudaEventRecord(b->staged, s)) != cudaSuccess)
         return qtk::cuda_error((int)e, "batch upload");
 
-    const int kind = (ncoop < tiles.size() ? 1 : 0) | (ncoop ? 2 : 0);
-    if (!b->exec[kind])
-        if (int rc = capture(b, kind)) return rc;
-    if ((e = cudaGraphLaunch(b->exec[kind], s)) != cudaSuccess) return qtk::cuda_error((int)e, "graph launch");
+    if (!b->exec.count(kinds))
+        if (int rc = build_graph(b, kinds)) return rc;
+    if ((e = cudaGraphLaunch(b->exec[kinds], s)) != cudaSuccess) return qtk::cuda_error((int)e, "graph launch");
     if ((e = cudaEventRecord(b->done, s)) != cudaSuccess) return qtk::cuda_error((int)e, "graph launch");
     return QT_OK;
 }

@@ -885,8 +885,8 @@ __global__ void __launch_bounds__(tpb::kThreads, kCoopSearchCtas) k_bc1_coop_sea
     coop_search_queue<IT, K_TB>(2, rgba, w, h, bw, p.search_rounds, out, bc3, aligned, q, f);
 }
 
-// The batch's tiles whose textures run cooperatively (coop_batch_setting): tiles[0 .. ctl[3]), claimed through ctl[2] as
-// k_batch claims the others. One texture per tile, so a warp's settings are uniform.
+// The batch's tiles whose textures run cooperatively (coop_batch_setting): tiles[.. ctl[1]), claimed through ctl[0] as k_batch
+// claims the others. One texture per tile, so a warp's settings are uniform.
 template <int IT> __device__ __noinline__ uint2 encode_warp_batch(const qt_bc1_params &p, int color_mode, bool have, int pp) {
     return coop::encode_warp<IT>(p, color_mode, have, pp);
 }
@@ -896,10 +896,10 @@ __global__ void __launch_bounds__(tpb::kThreads, 4) k_batch_coop(const BatchItem
     load_tables_smem();
     coop::load_fit_tables(true);
     const int lane = threadIdx.x & 31;
-    const uint32_t ntiles = ctl[3];
+    const uint32_t ntiles = ctl[1];
     while (true) {
         uint32_t t = 0;
-        if (lane == 0) t = atomicAdd(&ctl[2], 1u);
+        if (lane == 0) t = atomicAdd(&ctl[0], 1u);
         t = __shfl_sync(0xFFFFFFFFu, t, 0);
         if (t >= ntiles) break;
         const TileDev T = tiles[t];

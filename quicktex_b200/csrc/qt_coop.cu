@@ -121,15 +121,13 @@ void coop_defer_rest(const uint8_t *rgba, int w, int h, const qt_bc1_params &p, 
     });
 }
 
-int launch_batch_coop(const BatchItemDev *items, const TileDev *tiles, uint32_t *ctl, void *stream) {
+int batch_coop_launch(BatchLaunch *l) {
     static std::atomic<uint64_t> done{0};
     const cudaError_t e = allow_smem(k_batch_coop, coop::kFitSmem, done);
     if (e != cudaSuccess) return (int)e;
-    k_batch_coop<<<num_sms() * kCoopCtas, tpb::kThreads, coop::kFitSmem, (cudaStream_t)stream>>>(items, tiles, ctl);
-    return (int)cudaGetLastError();
+    *l = BatchLaunch{(const void *)k_batch_coop, num_sms() * kCoopCtas, tpb::kThreads, coop::kFitSmem};
+    return 0;
 }
-
-int batch_coop_warps() { return num_sms() * kCoopCtas * coop::kWarps; }
 
 cudaError_t upload_coop_tables() { return cudaMemcpyToSymbol(g_tab, &host_tables(), sizeof(DevTables)); }
 

@@ -119,11 +119,19 @@ int launch_batch(const BatchItemDev *items, const TileDev *tiles, uint32_t *ctl,
 // runs the same tiles); grid <= 0 fills the SMs to the kernel's occupancy at that size
 int launch_batch(const BatchItemDev *items, const TileDev *tiles, uint32_t *ctl, int grid, int threads, void *stream);
 int batch_ctas_per_sm();
-// Whether a batch's BC1/BC3 encode with these settings goes to the cooperative kernel, and that kernel: it pulls
-// tiles[0 .. ctl[3]) through the counter ctl[2]. batch_coop_warps: its resident warps.
+// A batch's kernels, each with its own range of tiles and its own pair of control words (head, end): 0 k_batch, 1 the
+// cooperative encoder, 2.. the specialised encoders. batch_kind: the one that runs an item; batch_launch: how to launch it
+// (0, or a cudaError_t).
+constexpr int kBatchKinds = 26;
+struct BatchLaunch {
+    const void *func;
+    int grid, threads;
+    size_t smem;
+};
+int batch_kind(int op, int fmt, const qt_bc1_params &p);
+int batch_launch(int kind, int ctas_per_sm, int threads, BatchLaunch *l);
+int batch_coop_launch(BatchLaunch *l);
 bool coop_batch_setting(const qt_bc1_params &p);
-int launch_batch_coop(const BatchItemDev *items, const TileDev *tiles, uint32_t *ctl, void *stream);
-int batch_coop_warps();
 int batch_sms();
 
 }  // namespace qtk
