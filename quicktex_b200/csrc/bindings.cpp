@@ -140,6 +140,11 @@ struct NoFill {};
 class Texture {
    public:
     virtual ~Texture() = default;
+    // the destructor alone would leave only the copies: a result returned by value then copied its texels (250 us at 1024^2)
+    Texture(const Texture &) = default;
+    Texture(Texture &&) noexcept = default;
+    Texture &operator=(const Texture &) = default;
+    Texture &operator=(Texture &&) noexcept = default;
     int Width() const { return w_; }
     int Height() const { return h_; }
     std::tuple<int, int> Size() const { return {w_, h_}; }

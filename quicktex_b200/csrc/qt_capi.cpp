@@ -532,6 +532,12 @@ class HostCache {
         *out = p;
         return QT_OK;
     }
+    // whether [p, p + n) lies in one pinned block that starts at p (a texture's storage does)
+    bool pinned(const void *p, size_t n) {
+        std::lock_guard<std::mutex> lk(mu_);
+        const auto it = live_.find(const_cast<void *>(p));
+        return it != live_.end() && it->second.pinned && n <= it->second.cls;
+    }
     void release(void *p) {
         if (!p) return;
         void *drop = nullptr;
@@ -603,6 +609,44 @@ struct HostXfer {
     int finish() { return st ? st->flush() : QT_OK; }
 };
 
+// Host path of a small texture: the kernel reads and writes pinned host memory over the link itself, one launch and one wait
+// in place of two copies around it. For launches that read each texel once (fewer than kDirectBlocks blocks: no split pass).
+// Buffers are the library's own pinned blocks (their size is known) or, for pageable memory, chunks of the thread's
+// staging ring; *done stays false for memory pinned elsewhere, whose extent is not known here. BC1 level 5 at 256^2, drop-in:
+// encode 51 -> 37 us, decode 36 -> 26
+// (the texels of a result moved in both).
+constexpr long kDirectBlocks = 16384;
+template <typename Launch>
+int run_host_direct(const uint8_t *src, size_t src_bytes, uint8_t *dst, size_t dst_bytes, Launch &&launch, const char *what, bool *done) {
+    const bool in_own = HostCache::get().pinned(src, src_bytes), out_own = HostCache::get().pinned(dst, dst_bytes);
+    *done = (in_own || is_pageable(src)) && (out_own || is_pageable(dst));
+    if (!*done) return QT_OK;
+    int dev = 0, rc, j;
+    if ((rc = ensure_device(&dev))) return rc;
+    const uint8_t *in = src;
+    uint8_t *out = dst;
+    if (!in_own || !out_own) {
+        Stage &st = thread_stage(dev);
+        if ((rc = st.init())) return rc;
+        if (!in_own) {
+            if ((rc = st.take(&j))) return rc;
+            CopyPool::get().copy(st.chunk(j), src, src_bytes);
+            in = st.chunk(j);
+        }
+        if (!out_own) {
+            if ((rc = st.take(&j))) return rc;
+            out = st.chunk(j);
+        }
+    }
+    cudaStream_t s = thread_stream(dev);
+    if ((rc = launch(in, out, (void *)s))) rc = cuda_err((cudaError_t)rc, what);
+    const cudaError_t e = cudaStreamSynchronize(s);
+    if (rc) return rc;
+    if (e != cudaSuccess) return cuda_err(e, what);
+    if (!out_own) CopyPool::get().copy(dst, out, dst_bytes);
+    return QT_OK;
+}
+
 // host path: H2D, kernel, D2H on this thread's stream; returns when done
 template <typename Launch>
 int run_host(const void *src, size_t src_bytes, void *dst, size_t dst_bytes, bool dst_needs_zero, Launch &&launch,
@@ -671,6 +715,12 @@ int run_host_banded(const uint8_t *src, uint8_t *dst, bool encode, int w, int h,
     const int nbands = (int)cut.size() - 1;
     const bool ragged = (h & 3) != 0;
     const size_t in_bytes = encode ? texel_bytes : blocks_bytes, out_bytes = encode ? blocks_bytes : texel_bytes;
+    if ((long)bw * bh < kDirectBlocks) {
+        bool done = false;
+        const int drc = run_host_direct(src, in_bytes, dst, out_bytes,
+                                        [&](const void *in, void *out, void *st) { return launch(const_cast<void *>(in), out, 0L, (long)bw * bh, st); }, what, &done);
+        if (done) return drc;
+    }
     if (nbands < 2 || (!encode && ragged))
         return run_host(src, in_bytes, dst, out_bytes, false,
                         [&](void *in, void *out, void *st) { return launch(in, out, 0L, (long)bw * bh, st); }, what);
