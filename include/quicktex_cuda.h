@@ -168,9 +168,9 @@ int qt_bc5_decode_device(const uint8_t *blocks, int width, int height, int chan0
  *
  * Many textures of any size, format and level in one launch: every texture is
  * cut into tiles of consecutive blocks (tile size per format/level from a tuning
- * table), the tiles are queued heaviest-first in device memory, and one
- * persistent kernel, replayed from a captured CUDA graph, pulls tiles until the
- * queue is empty. Each texture's output is byte-identical to the single-texture
+ * table), the tiles are queued heaviest-first in device memory, and
+ * persistent kernels, one per kind of work in the run and replayed from a captured
+ * CUDA graph, pull tiles until the queue is empty. Each texture's output is byte-identical to the single-texture
  * entry points above. */
 #define QT_OP_ENCODE 0
 #define QT_OP_DECODE 1

@@ -21,10 +21,10 @@ namespace qtk {
 // the Full error mode and EndpointSearch (levels 13-19), and by what one block per lane would make of the
 // texture. Below ~75k blocks (a lane each) that mapping takes the time of one block's chain of trials whatever
 // n is, and the cooperative one is faster the longer the chain: four-colour Ideal, level 13 at 128^2 44 -> 25 us, 256^2 43 -> 41,
-// 384^2 44 -> 46; level 15 at 256^2 60 -> 43, 512^2 69 -> 68, 768^2 80 -> 99; level 18 at 128^2 226 -> 45, 512^2 245 -> 106. On full lanes
+// 384^2 44 -> 46; level 15 at 256^2 60 -> 43, 512^2 69 -> 68, 768^2 80 -> 99; level 18 at 128^2 228 -> 46, 512^2 245 -> 106. On full lanes
 // it wins where a pass has enough trials to pay for a block's fixed part (~110 warp instructions a pass): level 16 at 1536^2
-// 435 -> 363 us, 2048^2 758 -> 743 (three-colour), 3000^2 1123 -> 1195; level 17 at 2048^2 789 -> 664, 3000^2 1704 -> 1744
-// (three-colour + black, AMD); level 18 at 4096^2 3697 -> 3333. Nvidia's palettes cost more to form and its searches
+// 435 -> 363 us, 2048^2 753 -> 746 (three-colour), 3000^2 1123 -> 1195; level 17 at 2048^2 792 -> 642, 3000^2 1704 -> 1744
+// (three-colour + black, AMD); level 18 at 4096^2 3693 -> 3226. Nvidia's palettes cost more to form and its searches
 // improve more often, so its lines lie lower: level 17 at 512^2 186 -> 157, 768^2 231 -> 257; level 18 at 768^2 316 -> 289, 1536^2 1345 ->
 // 1343 (three-colour + black), 3000^2 2179 -> 2231.
 bool coop_setting(const qt_bc1_params &p, long n) {

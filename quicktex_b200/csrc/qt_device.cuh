@@ -13,6 +13,7 @@
 
 #include <cfloat>
 #include <climits>
+#include <cstddef>
 #include <cstdint>
 
 #include "qt_internal.h"
@@ -29,16 +30,18 @@ struct DevTables {
     uint16_t hash3[256];
     float4 factors4[969];
     float4 factors3[153];
-    uint4 ord4[969];
-    uint4 ord3[153];
-    uint16_t coop4[969 * 128];
-    uint16_t coop3[153 * 32];
     uint32_t orders4[969];
     uint32_t orders3[153];
     uint32_t match5[4][256];
     uint32_t match6[4][256];
+    uint4 ord4[969];
+    uint4 ord3[153];
+    uint16_t coop4[969 * 128];
+    uint16_t coop3[153 * 32];
 };
-static_assert(sizeof(DevTables) == sizeof(HostTables), "device and host table images must match");
+static_assert(sizeof(DevTables) == sizeof(HostTables) && offsetof(DevTables, ord4) == offsetof(HostTables, ord4) &&
+                  offsetof(DevTables, coop3) == offsetof(HostTables, coop3),
+              "device and host table images must match");
 
 static __device__ DevTables g_tab;
 

@@ -19,14 +19,15 @@ struct alignas(16) HostTables {
     uint16_t hash3[256];
     float factors4[969][4];     // 2x2 LS inverse per ordering (OrderTable.h:65-83)
     float factors3[153][4];
-    uint32_t ord4[969][4];      // cooperative fit: factors x, y (= z), w as bits; byte offsets 8 h0, 8 (h0 + h1), 8 (h0 + h1 + h2)
-    uint32_t ord3[153][4];      // ... 8 h0, 8 (h0 + h1)
-    uint16_t coop4[969 * 128];  // best4 as the cooperative fit reads it: within each 32, ordered for the shared memory's banks
-    uint16_t coop3[153 * 32];   // (ordering | 1 << 10 for a single colour | place within its 32 << 11)
     uint32_t orders4[969];      // histogram bytes h0 | h1<<8 | h2<<16 | h3<<24
     uint32_t orders3[153];
     uint32_t match5[4][256];    // single-colour tables per interpolator: high | low<<8 | err<<16
     uint32_t match6[4][256];
+    // last, so that the tables that one block per lane reads lie together
+    alignas(16) uint32_t ord4[969][4];      // cooperative fit: factors x, y (= z), w as bits; byte offsets 8 h0, 8 (h0 + h1), 8 (h0 + h1 + h2)
+    uint32_t ord3[153][4];      // ... 8 h0, 8 (h0 + h1)
+    uint16_t coop4[969 * 128];  // best4 as the cooperative fit reads it: within each 32, ordered for the shared memory's banks
+    uint16_t coop3[153 * 32];   // (ordering | 1 << 10 for a single colour | place within its 32 << 11)
 };
 
 // Device descriptor of one texture of a batch (built from qt_batch_item).

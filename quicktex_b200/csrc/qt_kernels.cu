@@ -15,8 +15,10 @@
 // result is an integer below 2^24, i.e. exact.
 //
 // BC4/BC5 encode and all decoders are HBM-bound: one thread per block,
-// 16-byte row loads/stores where the texture is 4-aligned. The persistent
-// batch kernel (k_batch) runs any mix of them from a device work queue.
+// 16-byte row loads/stores where the texture is 4-aligned, 32-bit words elsewhere.
+// The persistent batch kernels (k_batch: any mix; k_batch_fast: BC1/BC3 without a
+// search) run tiles from a device work queue. The cooperative encoder of levels
+// 13-19 is in qt_coop.cu.
 
 #include <cuda_pipeline.h>
 #include <cuda_runtime.h>
@@ -532,6 +534,12 @@ static DeferQueues defer_layout(uint32_t *scratch, long n, bool cf2) {
     return d;
 }
 
+template <int IT>
+static void launch_split(cudaStream_t s, const uint8_t *rgba, int w, int h, long b0, long b1, uint8_t *out, bool bc3, int aligned, uint32_t *list,
+                         uint32_t *count) {
+    k_bc1_split<IT><<<grid_for(b1 - b0, kSplitThreads), kSplitThreads, 0, s>>>(rgba, w, h, (w + 3) / 4, b0, b1, out, bc3, aligned, list, count);
+}
+
 // The deferred path's first passes over the blocks [b0, b1): the split pass lists the
 // non-solid blocks in list/count, the encoder runs each to its first cluster-fit pass and
 // queues what remains (second pass, 3-colour trials, EndpointSearch) in d.
@@ -540,7 +548,7 @@ static void defer_front(const uint8_t *rgba, int w, int h, const qt_bc1_params &
                         const DeferQueues &d, bool coop, uint32_t *list, uint32_t *count, long b0, long b1, cudaStream_t s) {
     const int bw = (w + 3) / 4;
     const long n = b1 - b0;
-    k_bc1_split<I><<<grid_for(n, 256), 256, 0, s>>>(rgba, w, h, bw, b0, b1, out, bc3, aligned, list, count);
+    launch_split<I>(s, rgba, w, h, b0, b1, out, bc3, aligned, list, count);
     if (coop) {
         coop_defer(rgba, w, h, p, out, bc3, aligned, n, list, count, d, s);
         return;
@@ -670,38 +678,36 @@ int launch_bc1_encode_range(const uint8_t *rgba, int w, int h, const qt_bc1_para
             });
             e = cudaGetLastError();
         } else if (e == cudaSuccess && p.search_rounds == 0) {
-            const int gs = grid_for(n, 256);
             switch (p.interpolator) {
-                case IT_IDEAL: k_bc1_split<IT_IDEAL><<<gs, 256, 0, s>>>(rgba, w, h, bw, b_begin, b_end, out, bc3, aligned, list, count); break;
-                case IT_ROUND: k_bc1_split<IT_ROUND><<<gs, 256, 0, s>>>(rgba, w, h, bw, b_begin, b_end, out, bc3, aligned, list, count); break;
-                case IT_NVIDIA: k_bc1_split<IT_NVIDIA><<<gs, 256, 0, s>>>(rgba, w, h, bw, b_begin, b_end, out, bc3, aligned, list, count); break;
-                default: k_bc1_split<IT_AMD><<<gs, 256, 0, s>>>(rgba, w, h, bw, b_begin, b_end, out, bc3, aligned, list, count); break;
+                case IT_IDEAL: launch_split<IT_IDEAL>(s, rgba, w, h, b_begin, b_end, out, bc3, aligned, list, count); break;
+                case IT_ROUND: launch_split<IT_ROUND>(s, rgba, w, h, b_begin, b_end, out, bc3, aligned, list, count); break;
+                case IT_NVIDIA: launch_split<IT_NVIDIA>(s, rgba, w, h, b_begin, b_end, out, bc3, aligned, list, count); break;
+                default: launch_split<IT_AMD>(s, rgba, w, h, b_begin, b_end, out, bc3, aligned, list, count); break;
             }
             launch_fast(g, s, rgba, w, h, bw, 0, 0, p, out, bc3, aligned, list, count);
             e = cudaGetLastError();
         } else if (e == cudaSuccess && coop_setting(p, n)) {
             by_interp(p.interpolator, [&](auto I) {
                 constexpr int IT = decltype(I)::value;
-                k_bc1_split<IT><<<grid_for(n, 256), 256, 0, s>>>(rgba, w, h, bw, b_begin, b_end, out, bc3, aligned, list, count);
+                launch_split<IT>(s, rgba, w, h, b_begin, b_end, out, bc3, aligned, list, count);
             });
             e = coop_encode(rgba, w, h, 0, n, p, out, bc3, aligned, list, count, s);
         } else if (e == cudaSuccess) {
-            const int gs = grid_for(n, 256);
             switch (p.interpolator) {
                 case IT_IDEAL:
-                    k_bc1_split<IT_IDEAL><<<gs, 256, 0, s>>>(rgba, w, h, bw, b_begin, b_end, out, bc3, aligned, list, count);
+                    launch_split<IT_IDEAL>(s, rgba, w, h, b_begin, b_end, out, bc3, aligned, list, count);
                     k_bc1_thread<IT_IDEAL, true><<<g, tpb::kThreads, 0, s>>>(rgba, w, h, bw, 0, 0, p, out, bc3, aligned, list, count);
                     break;
                 case IT_ROUND:
-                    k_bc1_split<IT_ROUND><<<gs, 256, 0, s>>>(rgba, w, h, bw, b_begin, b_end, out, bc3, aligned, list, count);
+                    launch_split<IT_ROUND>(s, rgba, w, h, b_begin, b_end, out, bc3, aligned, list, count);
                     k_bc1_thread<IT_ROUND, true><<<g, tpb::kThreads, 0, s>>>(rgba, w, h, bw, 0, 0, p, out, bc3, aligned, list, count);
                     break;
                 case IT_NVIDIA:
-                    k_bc1_split<IT_NVIDIA><<<gs, 256, 0, s>>>(rgba, w, h, bw, b_begin, b_end, out, bc3, aligned, list, count);
+                    launch_split<IT_NVIDIA>(s, rgba, w, h, b_begin, b_end, out, bc3, aligned, list, count);
                     k_bc1_thread<IT_NVIDIA, true><<<g, tpb::kThreads, 0, s>>>(rgba, w, h, bw, 0, 0, p, out, bc3, aligned, list, count);
                     break;
                 default:
-                    k_bc1_split<IT_AMD><<<gs, 256, 0, s>>>(rgba, w, h, bw, b_begin, b_end, out, bc3, aligned, list, count);
+                    launch_split<IT_AMD>(s, rgba, w, h, b_begin, b_end, out, bc3, aligned, list, count);
                     k_bc1_thread<IT_AMD, true><<<g, tpb::kThreads, 0, s>>>(rgba, w, h, bw, 0, 0, p, out, bc3, aligned, list, count);
                     break;
             }
