@@ -85,18 +85,18 @@ BC1_DRAM_BYTES_PER_BLOCK = (16792832 + 18021376 + 2560 + 20707584 + 21565952 + 1
 # Warp instructions executed per block by one encode call of each setting: smsp__inst_executed.sum
 # over the call's kernels divided by the texture's blocks, from the ncu launch list of the bench's
 # own per-setting pass at 2048x2048 (a crop of the same texture, the same kernels: split + fast
-# encoder, or the five-kernel level-18 pipeline), summarised in
+# encoder, or the five-kernel level-18 pipelines), summarised in
 # profiles/bench_2048sq_inst_per_block.md.
 WARP_INST_PER_BLOCK: dict = {
-    "L0_four_ideal": 121.0, "L0_four_round": 121.7, "L0_four_nvidia": 122.8, "L0_four_amd": 120.8,
+    "L0_four_ideal": 120.9, "L0_four_round": 121.7, "L0_four_nvidia": 122.8, "L0_four_amd": 120.8,
     "L0_three_ideal": 188.3, "L0_three_round": 189.0, "L0_three_nvidia": 191.1, "L0_three_amd": 188.2,
-    "L0_three_black_ideal": 190.1, "L0_three_black_round": 190.8, "L0_three_black_nvidia": 192.8, "L0_three_black_amd": 189.9,
-    "L10_four_ideal": 443.9, "L10_four_round": 448.0, "L10_four_nvidia": 457.8, "L10_four_amd": 442.6,
-    "L10_three_ideal": 593.0, "L10_three_round": 597.1, "L10_three_nvidia": 612.6, "L10_three_amd": 591.7,
+    "L0_three_black_ideal": 190.0, "L0_three_black_round": 190.8, "L0_three_black_nvidia": 192.8, "L0_three_black_amd": 189.9,
+    "L10_four_ideal": 443.9, "L10_four_round": 448.0, "L10_four_nvidia": 457.8, "L10_four_amd": 442.5,
+    "L10_three_ideal": 593.0, "L10_three_round": 597.1, "L10_three_nvidia": 612.6, "L10_three_amd": 591.6,
     "L10_three_black_ideal": 594.8, "L10_three_black_round": 598.9, "L10_three_black_nvidia": 614.2, "L10_three_black_amd": 593.4,
-    "L18_four_ideal": 3221.0, "L18_four_round": 3266.3, "L18_four_nvidia": 3678.5, "L18_four_amd": 3225.4,
-    "L18_three_ideal": 3917.7, "L18_three_round": 3962.8, "L18_three_nvidia": 4511.4, "L18_three_amd": 3922.0,
-    "L18_three_black_ideal": 3917.9, "L18_three_black_round": 3963.0, "L18_three_black_nvidia": 4515.0, "L18_three_black_amd": 3924.5,
+    "L18_four_ideal": 2198.2, "L18_four_round": 2184.0, "L18_four_nvidia": 3677.8, "L18_four_amd": 2254.2,
+    "L18_three_ideal": 2821.7, "L18_three_round": 2807.5, "L18_three_nvidia": 4507.3, "L18_three_amd": 2877.0,
+    "L18_three_black_ideal": 2821.8, "L18_three_black_round": 2807.6, "L18_three_black_nvidia": 4507.5, "L18_three_black_amd": 2877.1,
 }
 
 
