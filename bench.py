@@ -77,10 +77,10 @@ CONFIG = {
 
 
 # DRAM bytes per block of a level-18 encode call (split, encoder, second cluster-fit pass, search,
-# finish), the setting class that holds ~80% of the step: the ncu capture summarised in
-# profiles/k_bc1_L18_2048sq_pipeline.md (dram__bytes_read.sum + dram__bytes_write.sum of the five
-# kernels = 92,676,096 B for 262,144 blocks). Each pass re-reads the block's texels.
-BC1_DRAM_BYTES_PER_BLOCK = (16792832 + 18021376 + 2560 + 20707584 + 21565952 + 15585792) / 262144
+# finish), the setting class that holds ~80% of the step: the ncu capture of the cooperative kernels
+# in profiles/k_bc1_L18_2048sq_pipeline.md (dram__bytes_read.sum + dram__bytes_write.sum of the five
+# kernels, 262,144 blocks, three-colour + black, IdealRound). Each pass re-reads the block's texels.
+BC1_DRAM_BYTES_PER_BLOCK = (16794112 + 18508288 + 23063552 + 21548544 + 15494400) / 262144
 
 # Warp instructions executed per block by one encode call of each setting: smsp__inst_executed.sum
 # over the call's kernels divided by the texture's blocks, from the ncu launch list of the bench's
@@ -328,7 +328,7 @@ def roofline_line(issue, achieved_exec, achieved_ref, peak_tops, sms, peaks_kind
             "traffic_source": "ncu dram bytes of the five kernels of one 2048^2 level-18 call, per block, "
                               "times this texture's blocks",
             "kernel": "BC1 encode call: qtk::k_bc1_split, then qtk::k_bc1_fast for settings without "
-                      "EndpointSearch, or qtk::k_bc1_defer + qtk::k_bc1_cf2 + qtk::k_bc1_search + qtk::k_bc1_finish",
+                      "EndpointSearch, or qtk::k_bc1_coop_defer + qtk::k_bc1_coop_cf2 + qtk::k_bc1_coop_search (Nvidia: qtk::k_bc1_defer + qtk::k_bc1_cf2 + qtk::k_bc1_search) + qtk::k_bc1_finish",
             "work_model": work}
     if issue:
         line.update({k: issue[k] for k in ("achieved", "peak", "unit", "frac", "by_level_frac", "source")})
