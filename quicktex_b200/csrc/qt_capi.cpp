@@ -614,12 +614,14 @@ struct HostXfer {
 // Buffers are the library's own pinned blocks (their size is known) or, for pageable memory, chunks of the thread's
 // staging ring; *done stays false for memory pinned elsewhere, whose extent is not known here. BC1 level 5 at 256^2, drop-in:
 // encode 51 -> 37 us, decode 36 -> 26
-// (the texels of a result moved in both).
+// (the texels of a result moved in both). A call whose source and destination share memory is staged: the kernel's
+// CTAs would write blocks over texels that others have yet to read.
 constexpr long kDirectBlocks = 16384;
 template <typename Launch>
 int run_host_direct(const uint8_t *src, size_t src_bytes, uint8_t *dst, size_t dst_bytes, Launch &&launch, const char *what, bool *done) {
     const bool in_own = HostCache::get().pinned(src, src_bytes), out_own = HostCache::get().pinned(dst, dst_bytes);
-    *done = (in_own || is_pageable(src)) && (out_own || is_pageable(dst));
+    const bool shared = src < dst + dst_bytes && dst < src + src_bytes;
+    *done = !shared && (in_own || is_pageable(src)) && (out_own || is_pageable(dst));
     if (!*done) return QT_OK;
     int dev = 0, rc, j;
     if ((rc = ensure_device(&dev))) return rc;

@@ -74,6 +74,31 @@ def test_every_kind_of_memory(w, h, src_kind, dst_kind):
         assert np.array_equal(out, tex.cpu().numpy()), (fmt, "decode")
 
 
+@pytest.mark.parametrize("fmt,w,h", [(1, 508, 512), (3, 512, 508), (4, 254, 260), (5, 505, 509)])
+def test_in_place(fmt, w, h):
+    """One block of memory as both source and destination: every texel is read before the first block is written over it (and
+    the other way round), as with buffers of their own."""
+    L, v = capi.lib(), capi._vp
+    img = np.ascontiguousarray(syn.alpha_mix(w, h, workload=18, stream=w + h)[:h, :w]).reshape(-1)
+    n = capi.nblocks(w, h) * (16 if fmt in (3, 5) else 8)
+    p = ctypes.byref(capi.params_for_level(18))
+    enc = {1: lambda s, d: L.qt_bc1_encode_host(s, w, h, p, d), 3: lambda s, d: L.qt_bc3_encode_host(s, w, h, p, d),
+           4: lambda s, d: L.qt_bc4_encode_host(s, w, h, 1, d), 5: lambda s, d: L.qt_bc5_encode_host(s, w, h, 2, 0, d)}[fmt]
+    dec = {1: lambda s, d: L.qt_bc1_decode_host(s, w, h, 0, 1, d), 3: lambda s, d: L.qt_bc3_decode_host(s, w, h, 0, d),
+           4: lambda s, d: L.qt_bc4_decode_host(s, w, h, 1, d), 5: lambda s, d: L.qt_bc5_decode_host(s, w, h, 2, 0, d)}[fmt]
+    a, b, c = (np.zeros(max(img.size, n) + 1, np.uint8) for _ in range(3))
+    a[:img.size] = img
+    capi.check(enc(v(a.ctypes.data), v(b.ctypes.data)))
+    capi.check(dec(v(b.ctypes.data), v(c.ctypes.data)))
+    own = _Own(max(img.size, n))
+    at = v(own.a.ctypes.data)
+    own.a[:img.size] = img
+    capi.check(enc(at, at))
+    assert np.array_equal(own.a[:n], b[:n]), "encode"
+    capi.check(dec(at, at))
+    assert np.array_equal(own.a[:img.size], c[:img.size]), "decode"
+
+
 def test_results_keep_their_bytes(oracle_lib):
     img = syn.block_mix(260, 252, workload=18, stream=9)
     outs = [BC1Encoder(5).encode(qt.RawTexture.frombytes(img.tobytes(), 260, 252)) for _ in range(3)]
