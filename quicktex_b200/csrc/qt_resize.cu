@@ -334,7 +334,8 @@ __global__ void __cluster_dims__(kSplit, 1, 1) __launch_bounds__(256) k_resize_s
     cluster.sync();  // the others' reads of this CTA's shared memory
 }
 
-// up to this many source texels
+// up to this many source texels, and only between separate buffers: its CTAs read the source while others write the result,
+// where the two passes of the general path have read all of it before the first write
 constexpr long kSmallTexels = 512L * 512;
 
 bool small_resize(const Scale &h, const Scale &v) {
@@ -400,7 +401,8 @@ extern "C" int qt_resize_bilinear_device(const uint8_t *src, int w, int h, uint8
     }
     const bool need_h = dw != w, need_v = dh != h;
     const Scale sh(w, dw), sv(h, dh);
-    if (small_resize(sh, sv)) {
+    const bool shared = src < dst + (size_t)dw * dh * 4 && dst < src + (size_t)w * h * 4;
+    if (!shared && small_resize(sh, sv)) {
         resize_small(reinterpret_cast<const uint32_t *>(src), sh, sv, reinterpret_cast<uint32_t *>(dst), s);
         e = cudaGetLastError();
         return e == cudaSuccess ? QT_OK : qtk::cuda_error((int)e, "resize");

@@ -25,3 +25,19 @@ def test_equals_pillow(w, h, to):
     resize_device(src.data_ptr(), w, h, dst.data_ptr(), to[0], to[1], torch.cuda.current_stream().cuda_stream)
     ref = np.asarray(resize_no_premultiply(Image.fromarray(img, "RGBA"), to))
     assert np.array_equal(dst.cpu().numpy(), ref)
+
+
+@pytest.mark.parametrize("w,h,to", [(512, 512, (300, 200)), (500, 333, (400, 666)), (300, 200, (333, 600)), (700, 600, (350, 300))])
+def test_in_place(w, h, to):
+    """Both directions change: the result may lie over the source, at its start or further on."""
+    import torch
+    from PIL import Image
+
+    img = np.ascontiguousarray(syn.alpha_mix(w, h, workload=17, stream=w + 7 * h))
+    ref = np.asarray(resize_no_premultiply(Image.fromarray(img, "RGBA"), to))
+    s = torch.cuda.current_stream().cuda_stream
+    for at in (0, 4 * w):
+        buf = torch.zeros(at + 4 * max(w * h, to[0] * to[1]), dtype=torch.uint8, device="cuda")
+        buf[:img.size] = torch.from_numpy(img.reshape(-1)).cuda()
+        resize_device(buf.data_ptr(), w, h, buf.data_ptr() + at, to[0], to[1], s)
+        assert np.array_equal(buf.cpu().numpy()[at:at + ref.size], ref.reshape(-1)), at
