@@ -135,4 +135,8 @@ int batch_coop_launch(BatchLaunch *l);
 bool coop_batch_setting(const qt_bc1_params &p);
 int batch_sms();
 
+// Rules of a dispatch on their own, without a device (C linkage: the CPU tests call them).
+// Whether a resize between separate buffers runs as one launch.
+extern "C" int qtk_resize_is_small(int w, int h, int dw, int dh);
+
 }  // namespace qtk

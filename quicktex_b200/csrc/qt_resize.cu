@@ -334,12 +334,14 @@ __global__ void __cluster_dims__(kSplit, 1, 1) __launch_bounds__(256) k_resize_s
     cluster.sync();  // the others' reads of this CTA's shared memory
 }
 
-// up to this many source texels, and only between separate buffers: its CTAs read the source while others write the result,
+// up to this many source texels and this many in the result, and only between separate buffers: its CTAs read the source while others write the result,
 // where the two passes of the general path have read all of it before the first write
 constexpr long kSmallTexels = 512L * 512;
 
+// Sizes first: with at most kSmallTexels texels on either side, the layout's and the launch's 32-bit products are in range.
 bool small_resize(const Scale &h, const Scale &v) {
-    return (long)h.in_size * v.in_size <= kSmallTexels && (long)SmallLayout(h, v).words * 4 <= 46 * 1024;
+    return (long)h.in_size * v.in_size <= kSmallTexels && (long)h.out_size * v.out_size <= kSmallTexels &&
+           (long)SmallLayout(h, v).words * 4 <= 46 * 1024;
 }
 
 template <int G> void resize_small_g(const uint32_t *in, const Scale &h, const Scale &v, uint32_t *out, cudaStream_t s) {
@@ -386,6 +388,8 @@ void resample_v(const uint32_t *in, int w, uint32_t *out, int dh, const int2 *b,
 }
 
 }  // namespace
+
+extern "C" int qtk_resize_is_small(int w, int h, int dw, int dh) { return small_resize(Scale(w, dw), Scale(h, dh)); }
 
 extern "C" int qt_resize_bilinear_device(const uint8_t *src, int w, int h, uint8_t *dst, int dw, int dh, void *stream) {
     if (!src || !dst) return qtk::set_error(QT_ERR_ARG, "NULL buffer");
