@@ -41,3 +41,11 @@ def test_in_place(w, h, to):
         buf[:img.size] = torch.from_numpy(img.reshape(-1)).cuda()
         resize_device(buf.data_ptr(), w, h, buf.data_ptr() + at, to[0], to[1], s)
         assert np.array_equal(buf.cpu().numpy()[at:at + ref.size], ref.reshape(-1)), at
+
+
+@pytest.mark.parametrize("w,h,to", [(6144, 2, (1, 1)), (1, 6144, (1, 1)), (6144, 60, (1, 30)), (1999, 333, (1, 1)), (1999, 333, (7, 2)), (33, 4097, (33, 4001)),
+                                    (4099, 3, (1, 3)), (1086, 109, (66, 1)), (1000, 1000, (1, 1)), (3000, 1000, (46, 15)), (4, 65536, (4, 32768))])
+def test_many_taps(w, h, to):
+    """Weights whose sum is taken in another order than Pillow's: 6144 to 1 puts some on the boundary between two fixed-point
+    values ((j + 1/2) / 3072^2 * 2^22 is a half for 2j + 1 = 9), where the sum has to be taken again in Pillow's order."""
+    test_equals_pillow(w, h, to)
