@@ -351,14 +351,20 @@ __global__ void __cluster_dims__(kSplit, 1, 1) __launch_bounds__(256) k_resize_s
     cluster.sync();  // the others' reads of this CTA's shared memory
 }
 
-// up to this many source texels and this many in the result, and only between separate buffers: its CTAs read the source while others write the result,
-// where the two passes of the general path have read all of it before the first write
-constexpr long kSmallTexels = 512L * 512;
+// Which resizes run as one launch: between separate buffers only (its CTAs read the source while others write the result,
+// where the two passes of the general path have read all of it before the first write), and where the clusters have little to do.
+// Each computes the horizontal taps for itself, and every source row is read by the clusters of the ~2 output rows that need
+// it, so many rows or columns cost more than three launches: up to 128 rows (8 CTAs each: one wave) and 16384
+// texels of result, and 64 K source texels a cluster, which only 8 SMs read. Measured, one launch / general path: 128^2 ->
+// 64^2 6.4 / 13.0 us, 256^2 -> 64^2 8.0 / 12.6, 500^2 -> 125^2 14.6 / 12.6, 512^2 -> 256^2 28.9 / 12.6, 500^2 -> 1000^2
+// 205 / 17; 1024^2 from 300^2 214 / 17; 1086 x 109 -> 66 x 1 (118 K texels a cluster) 33 / 14.4, 510 x 334 -> 7 x 5 (48 K) 17.2 / 16.6.
+constexpr long kSmallTexels = 512L * 512, kSmallRows = 128, kSmallResult = 16384, kSmallRead = 65536;
 
-// Sizes first: with at most kSmallTexels texels on either side, the layout's and the launch's 32-bit products are in range.
+// The result's size first: with it bounded, the layout's and the launch's 32-bit products are in range.
 bool small_resize(const Scale &h, const Scale &v) {
-    return (long)h.in_size * v.in_size <= kSmallTexels && (long)h.out_size * v.out_size <= kSmallTexels &&
-           (long)SmallLayout(h, v).words * 4 <= 46 * 1024;
+    if ((long)h.in_size * v.in_size > kSmallTexels || v.out_size > kSmallRows || (long)h.out_size * v.out_size > kSmallResult) return false;
+    const long rows = v.in_size == v.out_size ? 1 : std::min(v.ksize, v.in_size);
+    return rows * h.in_size <= kSmallRead && (long)SmallLayout(h, v).words * 4 <= 46 * 1024;
 }
 
 template <int G> void resize_small_g(const uint32_t *in, const Scale &h, const Scale &v, uint32_t *out, cudaStream_t s) {
