@@ -27,16 +27,19 @@ namespace qtk {
 // (three-colour + black, AMD); level 18 at 4096^2 3693 -> 3226. Nvidia's palettes cost more to form and its searches
 // improve more often, so its lines lie lower: level 17 at 512^2 186 -> 157, 768^2 231 -> 257; level 18 at 768^2 316 -> 289, 1536^2 1345 ->
 // 1343 (three-colour + black), 3000^2 2179 -> 2231.
-bool coop_setting(const qt_bc1_params &p, long n) {
-    if (p.error_mode != EM_FULL || p.search_rounds == 0) return false;
-    const unsigned trials = (p.exhaustive ? 969u : p.orderings4) * (p.two_cf_passes ? 2u : 1u);
-    const bool nvidia = p.interpolator == IT_NVIDIA;
-    if (trials >= 200) return !nvidia || n < defer_min_blocks();
+// The deferred path (defer_min blocks and more) has no cooperative kernels for Nvidia: its first line, whatever the device's size.
+extern "C" int qtk_coop_rule(const qt_bc1_params *p, long n, long defer_min) {
+    if (p->error_mode != EM_FULL || p->search_rounds == 0) return false;
+    const unsigned trials = (p->exhaustive ? 969u : p->orderings4) * (p->two_cf_passes ? 2u : 1u);
+    const bool nvidia = p->interpolator == IT_NVIDIA;
+    if (nvidia && n >= defer_min) return false;
+    if (trials >= 200) return true;
     if (trials >= 100) return n <= (nvidia ? 20000 : 400000);
-    if (trials >= 72) return nvidia ? n <= 16384 : n < defer_min_blocks();
+    if (trials >= 72) return nvidia ? n <= 16384 : n < defer_min;
     if (trials >= 48) return n <= (nvidia ? 9216 : 16384);
     return n <= (nvidia ? 3000 : 5000);
 }
+bool coop_setting(const qt_bc1_params &p, long n) { return qtk_coop_rule(&p, n, defer_min_blocks()); }
 
 // The same for a texture of a batch, which shares full lanes with the others, and whose alternative (k_batch) runs the
 // second pass and the search on the lanes that need them.
@@ -89,6 +92,7 @@ cudaError_t coop_encode(const uint8_t *rgba, int w, int h, long b0, long n, cons
     }
 }
 
+// (never Nvidia: qtk_coop_rule)
 template <typename F> static void by_coop_interp(int interpolator, F &&f) {
     switch (interpolator) {
         case IT_IDEAL: f(std::integral_constant<int, IT_IDEAL>()); break;

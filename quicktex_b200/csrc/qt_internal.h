@@ -138,5 +138,7 @@ int batch_sms();
 // Rules of a dispatch on their own, without a device (C linkage: the CPU tests call them).
 // Whether a resize between separate buffers runs as one launch.
 extern "C" int qtk_resize_is_small(int w, int h, int dw, int dh);
+// Whether a BC1/BC3 texture of n blocks runs the cooperative encoder on a device whose deferred path starts at defer_min blocks.
+extern "C" int qtk_coop_rule(const qt_bc1_params *p, long n, long defer_min);
 
 }  // namespace qtk

@@ -1,5 +1,7 @@
 """CPU: rules that choose a kernel, at sizes no test runs and on devices no test has."""
 
+import ctypes
+
 import pytest
 
 from quicktex_b200 import capi
@@ -29,3 +31,25 @@ def test_resize_with_much_to_do_per_row_is_not_small(w, h, to):
 @pytest.mark.parametrize("w,h,to", [(128, 128, (64, 64)), (256, 256, (32, 32)), (500, 500, (62, 62)), (250, 167, (3, 2)), (64, 64, (1, 1))])
 def test_small_chains_stay_small(w, h, to):
     assert capi.lib().qtk_resize_is_small(w, h, *to) == 1
+
+
+def _coop(level, interp, n, defer_min):
+    p = capi.params_for_level(level, capi.FOUR_COLOR, interp)
+    return capi.lib().qtk_coop_rule(ctypes.byref(p), ctypes.c_long(n), ctypes.c_long(defer_min))
+
+
+@pytest.mark.parametrize("sms", [1, 10, 19, 20, 148])
+@pytest.mark.parametrize("level", range(13, 20))
+def test_deferred_nvidia_never_runs_cooperatively(sms, level):
+    """The deferred path (1024 blocks per SM and more) has cooperative kernels for the other interpolations only, so on a device of any
+    size Nvidia's textures that reach it stay with the one-block-per-lane kernels."""
+    defer_min = 1024 * sms
+    sizes = (defer_min, defer_min + 1, 16384, 20000, 400000, 1 << 24)
+    assert [n for n in sizes if n >= defer_min and _coop(level, capi.NVIDIA, n, defer_min)] == []
+
+
+def test_coop_rule_on_148_sms():
+    d = 1024 * 148
+    assert [_coop(18, i, d - 1, d) for i in range(4)] == [1, 1, 1, 1] and [_coop(18, i, d, d) for i in range(4)] == [1, 1, 0, 1]
+    assert [_coop(17, i, 20000, d) for i in range(4)] == [1, 1, 1, 1] and [_coop(17, i, 20001, d) for i in range(4)] == [1, 1, 0, 1]
+    assert [_coop(13, i, 5000, d) for i in range(4)] == [1, 1, 0, 1] and _coop(13, 0, 5001, d) == 0 and _coop(12, 0, 100, d) == 0
