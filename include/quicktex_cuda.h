@@ -219,7 +219,9 @@ size_t qt_batch_last_tiles(const qt_batch *b);
 int qt_batch_run_plain(const qt_batch_item *items, size_t n, void *stream);
 /* Size the queue for up to `items` textures and `tiles` tiles now, so that later
  * runs within those limits never reallocate it (a reallocation waits for the
- * device and re-captures the graph). Never shrinks the queue. */
+ * device and rebuilds the graph). Never shrinks the queue. The graph grows by
+ * the kernels that runs need: the first run of a format, interpolation, error or
+ * colour mode new to the batch builds it again (at most 26 times). */
 int qt_batch_reserve(qt_batch *b, size_t items, size_t tiles);
 
 /* Many copies in one call (serving front ends staging request payloads): one

@@ -9,13 +9,13 @@
 // tail), uploads the queue, and replays the graph. BC1/BC3 encodes go to kernels
 // of their own beside k_batch, in the same graph: the cooperative encoder
 // (levels 16-19) and encoders specialised by interpolator, error mode and
-// colour mode. A graph is built the first time a run holds that set of kernels,
-// and again when a queue buffer has to grow.
+// colour mode. The one graph holds a node for each kernel that a run has needed so far; a run
+// switches its own on and the others off.
+// It is built again when a run needs a kernel that it lacks, or a queue buffer has to grow.
 
 #include <algorithm>
 #include <cstdlib>
 #include <cstring>
-#include <map>
 #include <mutex>
 #include <vector>
 
@@ -75,7 +75,11 @@ struct qt_batch {
     uint32_t *d_ctl = nullptr, *h_ctl = nullptr;
     cudaEvent_t staged = nullptr;     // the last upload from the pinned staging buffers
     cudaEvent_t done = nullptr;       // the last persistent launch (the queue is in use until then)
-    std::map<uint32_t, cudaGraphExec_t> exec;  // by the set of kernels (bit k: kind k) that a run holds tiles for
+    cudaGraph_t graph = nullptr;      // the kernels of `built` (bit k: kind k), side by side
+    cudaGraphExec_t exec = nullptr;
+    cudaGraphNode_t node[qtk::kBatchKinds] = {};
+    uint32_t built = 0, enabled = 0;  // the graph's kernels, and those that the next replay runs
+    size_t graphs = 0;                // built so far
 
     qt_batch() {
         for (int op = 0; op < 2; op++)
@@ -101,13 +105,20 @@ namespace {
 constexpr size_t kMinTiles = 16384;
 constexpr size_t kCtlBytes = 2 * qtk::kBatchKinds * sizeof(uint32_t);
 
-void drop_graphs(qt_batch *b) {
-    for (auto &e : b->exec) cudaGraphExecDestroy(e.second);
-    b->exec.clear();
+// (nodes stay enabled in a replay that was launched before; the executable goes once that has run)
+void drop_graph(qt_batch *b) {
+    if (b->exec) {
+        cudaEventSynchronize(b->done);
+        cudaGraphExecDestroy(b->exec);
+    }
+    if (b->graph) cudaGraphDestroy(b->graph);
+    b->exec = nullptr;
+    b->graph = nullptr;
+    b->built = b->enabled = 0;
 }
 
 void free_buffers(qt_batch *b) {
-    drop_graphs(b);
+    drop_graph(b);
     cudaFree(b->d_items);
     cudaFree(b->d_tiles);
     cudaFreeHost(b->h_items);
@@ -138,10 +149,10 @@ int grow(qt_batch *b, size_t items, size_t tiles) {
     return QT_OK;
 }
 
-// Builds the graph of a run's launches, side by side (replays read the queue through fixed pointers): the kernels of `kinds`
+// Builds the graph of the kernels of `kinds`, side by side (replays read the queue through fixed pointers).
 int build_graph(qt_batch *b, uint32_t kinds) {
-    cudaGraph_t g = nullptr;
-    cudaError_t e = cudaGraphCreate(&g, 0);
+    drop_graph(b);
+    cudaError_t e = cudaGraphCreate(&b->graph, 0);
     for (int k = 0; k < qtk::kBatchKinds && e == cudaSuccess; k++) {
         if (!((kinds >> k) & 1u)) continue;
         qtk::BatchLaunch l;
@@ -154,19 +165,38 @@ int build_graph(qt_batch *b, uint32_t kinds) {
         np.blockDim = dim3((unsigned)l.threads);
         np.sharedMemBytes = (unsigned)l.smem;
         np.kernelParams = args;
-        cudaGraphNode_t node;
-        e = cudaGraphAddKernelNode(&node, g, nullptr, 0, &np);
+        e = cudaGraphAddKernelNode(&b->node[k], b->graph, nullptr, 0, &np);
         if (e == cudaSuccess && k == 1) {  // its tiles are the long ones: they start first
             cudaLaunchAttributeValue v = {};
             v.priority = -1;
-            e = cudaGraphKernelNodeSetAttribute(node, cudaLaunchAttributePriority, &v);
+            e = cudaGraphKernelNodeSetAttribute(b->node[k], cudaLaunchAttributePriority, &v);
         }
     }
-    cudaGraphExec_t exec = nullptr;
-    if (e == cudaSuccess) e = cudaGraphInstantiate(&exec, g, 0);
-    if (g) cudaGraphDestroy(g);
-    if (e != cudaSuccess) return qtk::cuda_error((int)e, "building the batch's graph");
-    b->exec[kinds] = exec;
+    if (e == cudaSuccess) e = cudaGraphInstantiate(&b->exec, b->graph, 0);
+    if (e != cudaSuccess) {
+        b->exec = nullptr;
+        drop_graph(b);
+        return qtk::cuda_error((int)e, "building the batch's graph");
+    }
+    b->built = b->enabled = kinds;
+    b->graphs++;
+    return QT_OK;
+}
+
+// The graph that runs exactly the kernels of `kinds`. One graph with switches, not one per set of kernels: a server's mixes
+// form ever new sets, and each would cost an instantiation (~0.2 ms) in a request's path and stay for good. It grows
+// by the kernels that runs need, at most kBatchKinds times, and does not start with all of them: 24 switched-off
+// kernels cost a run 6-20 us (BC1 level 0 at 64^2 65 -> 79 us, at 2048^2 138 -> 149).
+int use_graph(qt_batch *b, uint32_t kinds) {
+    if (kinds & ~b->built) {
+        if (int rc = build_graph(b, b->built | kinds)) return rc;
+    }
+    for (uint32_t change = kinds ^ b->enabled; change; change &= change - 1) {
+        const int k = __builtin_ctz(change);
+        const cudaError_t e = cudaGraphNodeSetEnabled(b->exec, b->node[k], (kinds >> k) & 1u);
+        if (e != cudaSuccess) return qtk::cuda_error((int)e, "switching the batch's kernels");
+        b->enabled ^= 1u << k;
+    }
     return QT_OK;
 }
 
@@ -193,6 +223,8 @@ int qtk::check_item_fields(const qt_batch_item &it) {
     if (it.op == QT_OP_ENCODE && (it.format == 1 || it.format == 3)) return qtk::check_bc1_params(&it.params, it.format == 3);
     return QT_OK;
 }
+
+extern "C" size_t qtk_batch_graphs(const qt_batch *b) { return b->graphs; }
 
 extern "C" {
 
@@ -255,7 +287,7 @@ int qt_batch_set_rules(qt_batch *b, const qt_tile_rule *rules, size_t n) {
 int qt_batch_set_grid(qt_batch *b, int ctas_per_sm) {
     if (!b || ctas_per_sm < 0) return qtk::set_error(QT_ERR_ARG, "invalid grid");
     std::lock_guard<std::mutex> lk(b->mu);
-    if (ctas_per_sm != b->ctas_per_sm) drop_graphs(b);
+    if (ctas_per_sm != b->ctas_per_sm) drop_graph(b);
     b->ctas_per_sm = ctas_per_sm;
     return QT_OK;
 }
@@ -264,7 +296,7 @@ int qt_batch_set_threads(qt_batch *b, int threads_per_cta) {
     if (!b || (threads_per_cta != 32 && threads_per_cta != 64 && threads_per_cta != 128))
         return qtk::set_error(QT_ERR_ARG, "threads per CTA must be 32, 64 or 128");
     std::lock_guard<std::mutex> lk(b->mu);
-    if (threads_per_cta != b->threads) drop_graphs(b);
+    if (threads_per_cta != b->threads) drop_graph(b);
     b->threads = threads_per_cta;
     return QT_OK;
 }
@@ -379,6 +411,7 @@ int qt_batch_run(qt_batch *b, const qt_batch_item *items, size_t n, void *stream
         b->h_ctl[2 * k + 1] = (uint32_t)i + 1;
         kinds |= 1u << k;
     }
+    if (int rc = use_graph(b, kinds)) return rc;
     cudaStream_t s = (cudaStream_t)stream;
     // runs on other streams: do not overwrite the queue before the previous launch finished reading it
     if ((e = cudaStreamWaitEvent(s, b->done, 0)) != cudaSuccess) return qtk::cuda_error((int)e, "batch ordering");
@@ -388,9 +421,7 @@ int qt_batch_run(qt_batch *b, const qt_batch_item *items, size_t n, void *stream
         (e = cudaEventRecord(b->staged, s)) != cudaSuccess)
         return qtk::cuda_error((int)e, "batch upload");
 
-    if (!b->exec.count(kinds))
-        if (int rc = build_graph(b, kinds)) return rc;
-    if ((e = cudaGraphLaunch(b->exec[kinds], s)) != cudaSuccess) return qtk::cuda_error((int)e, "graph launch");
+    if ((e = cudaGraphLaunch(b->exec, s)) != cudaSuccess) return qtk::cuda_error((int)e, "graph launch");
     if ((e = cudaEventRecord(b->done, s)) != cudaSuccess) return qtk::cuda_error((int)e, "graph launch");
     return QT_OK;
 }

@@ -135,10 +135,12 @@ int batch_coop_launch(BatchLaunch *l);
 bool coop_batch_setting(const qt_bc1_params &p);
 int batch_sms();
 
-// Rules of a dispatch on their own, without a device (C linkage: the CPU tests call them).
+// For the tests (C linkage). Rules of a dispatch on their own, without a device:
 // Whether a resize between separate buffers runs as one launch.
 extern "C" int qtk_resize_is_small(int w, int h, int dw, int dh);
 // Whether a BC1/BC3 texture of n blocks runs the cooperative encoder on a device whose deferred path starts at defer_min blocks.
 extern "C" int qtk_coop_rule(const qt_bc1_params *p, long n, long defer_min);
+// Graphs that a batch has built (one, and one more for each growth of its queue or of its set of kernels).
+extern "C" size_t qtk_batch_graphs(const qt_batch *b);
 
 }  // namespace qtk
