@@ -168,8 +168,8 @@ int qt_bc5_decode_device(const uint8_t *blocks, int width, int height, int chan0
  *
  * Many textures of any size, format and level in one launch: every texture is
  * cut into tiles of consecutive blocks (tile size per format/level from a tuning
- * table), the tiles are queued heaviest-first in device memory, and
- * persistent kernels, one per kind of work in the run and replayed from a captured
+ * table, smaller in a run too short to fill the GPU), the tiles are queued heaviest-first in device memory, and
+ * persistent kernels, one per kind of work in the run and replayed from a
  * CUDA graph, pull tiles until the queue is empty. Each texture's output is byte-identical to the single-texture
  * entry points above. */
 #define QT_OP_ENCODE 0
@@ -189,7 +189,7 @@ typedef struct qt_batch_item {
     int32_t write_alpha;   /* BC1 decode */
 } qt_batch_item;
 
-/* Tuning rule: tiles of `tile_blocks` blocks and a relative cost per block for
+/* Tuning rule: tiles of at most `tile_blocks` blocks and a relative cost per block for
  * (op, format, level); level is ignored for BC4/BC5 and decodes (-1). */
 typedef struct qt_tile_rule {
     int32_t op, format, level;

@@ -96,10 +96,13 @@ def tune(device: int = 0, quick: bool = False) -> dict:
         arena = Arena(_class_jobs(op, fmt, max(level, 0), budget, rng), device)
         arena.upload()
         nblocks = sum(j.nblocks for j in arena.jobs)
-        best = None
+        best, seen = None, set()
         for t in tiles:
             batch.set_rules([{"op": op, "format": fmt_id[fmt], "level": level, "tile_blocks": t, "cost_per_block": 1.0}])
             ms = _time(batch, arena)
+            if batch.last_tiles() in seen:  # the batch cut its tiles finer than t already: another measurement of the same tiles
+                break
+            seen.add(batch.last_tiles())
             if best is None or ms < best[1]:
                 best = (t, ms)
         measured.append({"op": op, "format": fmt_id[fmt], "level": level, "tile_blocks": best[0],

@@ -87,7 +87,7 @@ def load_tuning(path: str = TUNING_PATH) -> Optional[dict]:
 
 
 class Batch:
-    """One batch queue (device buffers + captured graph) on one device."""
+    """One batch queue (device buffers + graph of its kernels) on one device."""
 
     def __init__(self, device: int = 0, tuning: Optional[dict] = None, use_default_tuning: bool = True):
         self.device = device

@@ -101,8 +101,12 @@ struct qt_batch {
 
 namespace {
 
-// the queue's smallest capacity: a run's tiles are cut finer to fill the GPU only while they fit it
-constexpr size_t kMinTiles = 16384;
+constexpr size_t kMinTiles = 16384;  // the queue's smallest capacity
+
+// Warps that the kernels keep resident, and the most tiles that cutting a run finer than its rules (qt_batch_run) can add
+int resident_warps() { return qtk::batch_sms() * 16; }
+size_t finer_tiles(size_t items) { return 2 * (size_t)resident_warps() + items; }
+
 constexpr size_t kCtlBytes = 2 * qtk::kBatchKinds * sizeof(uint32_t);
 
 // (nodes stay enabled in a replay that was launched before; the executable goes once that has run)
@@ -321,7 +325,7 @@ int qt_batch_reserve(qt_batch *b, size_t items, size_t tiles) {
     int cur = 0;
     cudaGetDevice(&cur);
     if (cur != b->device) return qtk::set_error(QT_ERR_STATE, "qt_batch_reserve: the batch belongs to another device");
-    return grow(b, std::max<size_t>(items, b->cap_items), std::max<size_t>(tiles, b->cap_tiles));
+    return grow(b, std::max<size_t>(items, b->cap_items), std::max<size_t>(tiles + finer_tiles(items), b->cap_tiles));
 }
 
 int qt_batch_run(qt_batch *b, const qt_batch_item *items, size_t n, void *stream) {
@@ -340,7 +344,6 @@ int qt_batch_run(qt_batch *b, const qt_batch_item *items, size_t n, void *stream
     };
     std::vector<Plan> plan(n);
     double work[2] = {0, 0};  // of the kernels that run a block per lane, of the cooperative one
-    size_t coarse = 0;
     for (size_t i = 0; i < n; i++) {
         const qt_batch_item &it = items[i];
         if (int rc = check_item(it)) return rc;
@@ -365,14 +368,14 @@ int qt_batch_run(qt_batch *b, const qt_batch_item *items, size_t n, void *stream
         pl.rule = b->rules[rule_index(it.op, it.format, leveled ? qtk_level_of(it.params) : 0)];
         pl.kind = qtk::batch_kind(it.op, it.format, it.params);
         work[pl.kind == 1] += (double)pl.rule.cost * (double)nb;
-        coarse += (size_t)((nb + pl.rule.tile_blocks - 1) / pl.rule.tile_blocks);
     }
-    // Tiles of the rules' sizes, or smaller where the resident warps would have fewer than four each (a short batch
+    // Tiles of the rules' sizes, or smaller where the resident warps would have fewer than one each (a short batch
     // waits for its longest tile): a cooperative warp works on one block at a time, so its tiles may fall to a few
-    // blocks; the others keep 32, a block per lane.
-    const double warps = (double)qtk::batch_sms() * 16;
-    const size_t finer = 8 * (size_t)warps + n;
-    const bool cut = coarse + finer <= std::max(b->cap_tiles, kMinTiles);
+    // blocks; the others keep 32, a block per lane. The cut depends on this run's work alone. One tile per warp, not more: 1 / 2 / 4 of them take
+    // 176 / 214 / 322 us for 300 textures up to 256^2 (uncut 388) and 528 / 576 / 802 for 300 up to 1024^2 (uncut 559), where the
+    // host makes the tiles and the copy engine moves them. BC1 level 5 at 256^2 121 -> 41 us, its 64^2 chain 112 -> 30,
+    // level 18 at 256^2 285 -> 85, 20 mixed textures up to 256^2 363 -> 157, 200 up to 512^2 at levels 0-10 306 -> 149.
+    const double warps = resident_warps();
     struct Tile {
         int kind;
         float cost;
@@ -384,8 +387,9 @@ int qt_batch_run(qt_batch *b, const qt_batch_item *items, size_t n, void *stream
         const bool coop = pl.kind == 1;
         const uint64_t nb = (uint64_t)dev[i].bw * dev[i].bh;
         uint64_t tb = pl.rule.tile_blocks;
-        if (cut) {
-            const uint64_t fill = (uint64_t)(work[coop] / (warps * 4) / pl.rule.cost) + 1;
+        const double share = work[coop] / warps / pl.rule.cost;  // this texture's blocks in one warp's share of the run
+        if (share < (double)tb) {
+            const uint64_t fill = (uint64_t)share + 1;
             tb = std::min(tb, coop ? fill : (fill + 31) / 32 * 32);
         }
         for (uint64_t s0 = 0; s0 < nb; s0 += tb) {
