@@ -201,9 +201,13 @@ int qt_batch_create(int device, qt_batch **out);
 int qt_batch_destroy(qt_batch *b);
 /* Replace the tuning rules (rules not given keep their defaults). */
 int qt_batch_set_rules(qt_batch *b, const qt_tile_rule *rules, size_t n);
-/* Persistent grid size in CTAs per SM (0 = the kernel's occupancy limit). */
+/* Persistent grid size in CTAs per SM (0 = the kernel's occupancy limit). Below
+ * that limit (512 threads per SM) the batch holds no more of an SM than CTAs x
+ * threads at any time: all its kernels launch as many warps, one kernel after the
+ * other. From the limit on they run side by side, each with what it keeps resident. */
 int qt_batch_set_grid(qt_batch *b, int ctas_per_sm);
-/* Threads per CTA of the persistent kernel: 32, 64 or 128 (the default). Work is
+/* Threads per CTA: 32, 64 or 128 (the default), of the kernel that takes any tile;
+ * the specialised kernels form their CTAs from the same number of warps. Work is
  * claimed per warp, so the outputs do not depend on it. */
 int qt_batch_set_threads(qt_batch *b, int threads_per_cta);
 /* Enqueue one persistent launch over all items on `stream` (device buffers; the

@@ -125,11 +125,13 @@ void coop_defer_rest(const uint8_t *rgba, int w, int h, const qt_bc1_params &p, 
     });
 }
 
-int batch_coop_launch(BatchLaunch *l) {
+int batch_coop_launch(BatchLaunch *l, int *resident) {
     static std::atomic<uint64_t> done{0};
     const cudaError_t e = allow_smem(k_batch_coop, coop::kFitSmem, done);
     if (e != cudaSuccess) return (int)e;
-    *l = BatchLaunch{(const void *)k_batch_coop, num_sms() * kCoopCtas, tpb::kThreads, coop::kFitSmem};
+    l->func = (const void *)k_batch_coop;
+    l->smem = coop::kFitSmem;
+    *resident = kCoopCtas;
     return 0;
 }
 

@@ -119,7 +119,6 @@ int launch_batch(const BatchItemDev *items, const TileDev *tiles, uint32_t *ctl,
 // the same with `threads` per CTA (32, 64 or 128; work is claimed per warp, so any of them
 // runs the same tiles); grid <= 0 fills the SMs to the kernel's occupancy at that size
 int launch_batch(const BatchItemDev *items, const TileDev *tiles, uint32_t *ctl, int grid, int threads, void *stream);
-int batch_ctas_per_sm();
 // A batch's kernels, each with its own range of tiles and its own pair of control words (head, end): 0 k_batch, 1 the
 // cooperative encoder, 2.. the specialised encoders. batch_kind: the one that runs an item; batch_launch: how to launch it
 // (0, or a cudaError_t).
@@ -131,7 +130,8 @@ struct BatchLaunch {
 };
 int batch_kind(int op, int fmt, const qt_bc1_params &p);
 int batch_launch(int kind, int ctas_per_sm, int threads, BatchLaunch *l);
-int batch_coop_launch(BatchLaunch *l);
+int batch_coop_launch(BatchLaunch *l, int *resident);  // function and shared memory; CTAs that an SM holds
+bool batch_limited(int ctas_per_sm, int threads);       // the kernels of a batch run one after the other
 bool coop_batch_setting(const qt_bc1_params &p);
 int batch_sms();
 
@@ -142,5 +142,7 @@ extern "C" int qtk_resize_is_small(int w, int h, int dw, int dh);
 extern "C" int qtk_coop_rule(const qt_bc1_params *p, long n, long defer_min);
 // Graphs that a batch has built (one, and one more for each growth of its queue or of its set of kernels).
 extern "C" size_t qtk_batch_graphs(const qt_batch *b);
+// Pairs of its present graph's kernels of which the second waits for the first.
+extern "C" size_t qtk_batch_edges(const qt_batch *b);
 
 }  // namespace qtk

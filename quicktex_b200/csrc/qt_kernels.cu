@@ -751,24 +751,38 @@ int batch_kind(int op, int fmt, const qt_bc1_params &p) {
     return 2 + p.interpolator * 6 + (p.error_mode == EM_CHECK2 ? 3 : 0) + cm;
 }
 
+// A grid below k_batch's occupancy limit (ctas_per_sm * threads) leaves the rest of the SMs to other work: then every kernel of
+// the batch has that many warps per SM and no more (batch_limited: the kernels also run one after the other). Without one the kernels
+// other than k_batch launch what they keep resident, with the CTA size they were tuned at.
+bool batch_limited(int ctas_per_sm, int threads) {
+    return ctas_per_sm > 0 && ctas_per_sm * threads < batch_ctas_per_sm_at(tpb::kThreads) * tpb::kThreads;
+}
+
 int batch_launch(int kind, int ctas_per_sm, int threads, BatchLaunch *l) {
     *l = BatchLaunch{};
-    if (kind == 1) return batch_coop_launch(l);
+    if (threads != 32 && threads != 64 && threads != tpb::kThreads) return (int)cudaErrorInvalidValue;
     if (kind == 0) {
-        if (threads != 32 && threads != 64 && threads != tpb::kThreads) return (int)cudaErrorInvalidValue;
         l->func = (const void *)k_batch;
         l->threads = threads;
         l->grid = num_sms() * (ctas_per_sm > 0 ? ctas_per_sm : batch_ctas_per_sm_at(threads));
         return 0;
     }
-    const int k = (kind - 2) % 6, it = (kind - 2) / 6;
-    l->func = it == IT_IDEAL ? batch_fast_it<IT_IDEAL>(k) : it == IT_ROUND ? batch_fast_it<IT_ROUND>(k) : it == IT_NVIDIA ? batch_fast_it<IT_NVIDIA>(k) : batch_fast_it<IT_AMD>(k);
+    int resident = 5;  // CTAs per SM: 5 to 6 by the instance's registers
+    if (kind == 1) {
+        if (const int rc = batch_coop_launch(l, &resident)) return rc;
+    } else {
+        const int k = (kind - 2) % 6, it = (kind - 2) / 6;
+        l->func = it == IT_IDEAL ? batch_fast_it<IT_IDEAL>(k) : it == IT_ROUND ? batch_fast_it<IT_ROUND>(k) : it == IT_NVIDIA ? batch_fast_it<IT_NVIDIA>(k) : batch_fast_it<IT_AMD>(k);
+    }
     l->threads = tpb::kThreads;
-    l->grid = num_sms() * 5;  // resident CTAs per SM: 5 to 6 by the instance's registers
+    if (batch_limited(ctas_per_sm, threads)) {  // the same warps in the largest CTAs that divide them
+        const int lanes = ctas_per_sm * threads;
+        l->threads = lanes % tpb::kThreads == 0 ? tpb::kThreads : lanes % 64 == 0 ? 64 : 32;
+        resident = std::min(resident, lanes / l->threads);
+    }
+    l->grid = num_sms() * resident;
     return 0;
 }
-
-int batch_ctas_per_sm() { return batch_ctas_per_sm_at(tpb::kThreads); }
 
 int launch_batch(const BatchItemDev *items, const TileDev *tiles, uint32_t *ctl, int grid, int threads, void *stream) {
     // the kernel's shared-memory columns hold tpb::kThreads threads; smaller CTAs use a prefix
