@@ -154,15 +154,13 @@ int grow(qt_batch *b, size_t items, size_t tiles) {
 }
 
 // Builds the graph of the kernels of `kinds` (replays read the queue through fixed pointers): side by side, or one after the
-// other where the caller limited the grid, so that the batch holds no more of an SM at any time. The cooperative kernel comes
-// first: its tiles are the long ones.
+// other where the caller limited the grid, so that the batch holds no more of an SM at any time.
 int build_graph(qt_batch *b, uint32_t kinds) {
     drop_graph(b);
     const bool chain = qtk::batch_limited(b->ctas_per_sm, b->threads);
     int before = -1;
     cudaError_t e = cudaGraphCreate(&b->graph, 0);
-    for (int i = 0; i < qtk::kBatchKinds && e == cudaSuccess; i++) {
-        const int k = i < 2 ? 1 - i : i;
+    for (int k = 0; k < qtk::kBatchKinds && e == cudaSuccess; k++) {
         if (!((kinds >> k) & 1u)) continue;
         qtk::BatchLaunch l;
         if ((e = (cudaError_t)qtk::batch_launch(k, b->ctas_per_sm, b->threads, &l)) != cudaSuccess) break;
@@ -176,7 +174,7 @@ int build_graph(qt_batch *b, uint32_t kinds) {
         np.kernelParams = args;
         e = cudaGraphAddKernelNode(&b->node[k], b->graph, chain && before >= 0 ? &b->node[before] : nullptr, chain && before >= 0, &np);
         before = k;
-        if (e == cudaSuccess && k == 1) {
+        if (e == cudaSuccess && k == 1) {  // its tiles are the long ones: they start first
             cudaLaunchAttributeValue v = {};
             v.priority = -1;
             e = cudaGraphKernelNodeSetAttribute(b->node[k], cudaLaunchAttributePriority, &v);
