@@ -610,13 +610,12 @@ struct HostXfer {
 };
 
 // Host path of a small texture: the kernel reads and writes pinned host memory over the link itself, one launch and one wait
-// in place of two copies around it. For launches that read each texel once (fewer than kDirectBlocks blocks: no split pass).
+// in place of two copies around it, where that pays (qtk_host_direct).
 // Buffers are the library's own pinned blocks (their size is known) or, for pageable memory, chunks of the thread's
 // staging ring; *done stays false for memory pinned elsewhere, whose extent is not known here. BC1 level 5 at 256^2, drop-in:
 // encode 51 -> 37 us, decode 36 -> 26
 // (the texels of a result moved in both). A call whose source and destination share memory is staged: the kernel's
 // CTAs would write blocks over texels that others have yet to read.
-constexpr long kDirectBlocks = 16384;
 template <typename Launch>
 int run_host_direct(const uint8_t *src, size_t src_bytes, uint8_t *dst, size_t dst_bytes, Launch &&launch, const char *what, bool *done) {
     const bool in_own = HostCache::get().pinned(src, src_bytes), out_own = HostCache::get().pinned(dst, dst_bytes);
@@ -696,9 +695,10 @@ cudaEvent_t thread_event(int dev, int which = 0) {  // which < 3
 // bottom band, so it is not banded. launch(in, out, b_begin, b_end, stream) runs
 // the kernel over the blocks [b_begin, b_end).
 template <typename Launch>
-int run_host_banded(const uint8_t *src, uint8_t *dst, bool encode, int w, int h, size_t block_bytes, Launch &&launch,
+int run_host_banded(const uint8_t *src, uint8_t *dst, bool encode, int w, int h, int fmt, Launch &&launch,
                     const char *what, long min_band_blocks = 0) {
     const int bw = (w + 3) / 4, bh = (h + 3) / 4;
+    const size_t block_bytes = fmt == 3 || fmt == 5 ? 16 : 8;
     const size_t texel_row = (size_t)w * 4, block_row = (size_t)bw * block_bytes;
     const size_t texel_bytes = texel_row * (size_t)h, blocks_bytes = block_row * (size_t)bh;
     const size_t per_brow = 4 * texel_row + block_row;
@@ -717,7 +717,7 @@ int run_host_banded(const uint8_t *src, uint8_t *dst, bool encode, int w, int h,
     const int nbands = (int)cut.size() - 1;
     const bool ragged = (h & 3) != 0;
     const size_t in_bytes = encode ? texel_bytes : blocks_bytes, out_bytes = encode ? blocks_bytes : texel_bytes;
-    if ((long)bw * bh < kDirectBlocks) {
+    if (qtk::qtk_host_direct(encode, fmt, w, h)) {
         bool done = false;
         const int drc = run_host_direct(src, in_bytes, dst, out_bytes,
                                         [&](const void *in, void *out, void *st) { return launch(const_cast<void *>(in), out, 0L, (long)bw * bh, st); }, what, &done);
@@ -854,6 +854,25 @@ int set_error(int code, const char *msg) { return set_err(code, "%s", msg); }
 int cuda_error(int e, const char *what) { return cuda_err((cudaError_t)e, what); }
 int ensure_current_device(int *dev) { return ensure_device(dev); }
 int check_bc1_params(const qt_bc1_params *p, bool bc3) { return check_params(p, bc3); }
+
+// Fewer than 16384 blocks (a launch that reads each texel once: no split pass), and not where the link would carry many small
+// pieces. A decode writes a block's four rows one by one: in a narrow texture a warp's blocks lie in several block rows, and rows
+// off the 16-byte grid are written texel by texel. Decode of BC1 blocks, staged / direct: 8 x 24000 45 / 168 us, 64 x 3000 44 / 43,
+// 500 x 384 46 / 36; off the grid 33 x 7108 49 / 162, 125 x 1500 30 / 39, 191 x 1000 48 / 55, 301 x 600 47 / 41; 16-byte blocks
+// off the grid 33 x 7108 50 / 94, 129 x 1900 52 / 52. An encode reads rows, which the link
+// delivers in whole sectors: 12 x 20000 BC4 33 / 38; BC5 on the grid stages 16-byte pieces, half of them across a sector boundary where
+// the width is 4 modulo 8: 500 x 504 48 / 57, 480 x 528 47 / 38.
+extern "C" int qtk_host_direct(int encode, int fmt, int w, int h) {
+    const long n = (long)((w + 3) / 4) * ((h + 3) / 4);
+    if (n >= 16384) return false;
+    if (encode) {
+        if (fmt == 5 && w % 8 == 4) return n <= (w < 32 ? 4096 : 8192);
+        return w < 4 || w >= 16 || n <= 8192;
+    }
+    if (w % 4 == 0) return n <= 160L * w - 512;
+    if (fmt == 3 || fmt == 5) return w >= 125 || n <= (w < 32 ? 256 : 2048);
+    return w >= (w % 2 ? 193 : 176) || n <= (w < 32 ? 256 : w < 140 ? 512 : 4096);
+}
 
 cudaError_t scratch_alloc(void **ptr, size_t bytes, cudaStream_t stream) {
     int dev = 0;
@@ -1048,7 +1067,7 @@ int qt_bc1_encode_host(const uint8_t *rgba, int w, int h, const qt_bc1_params *p
     const qt_bc1_params pp = *p;
     if (qtk::bc1_parts_eligible((long)((w + 3) / 4) * ((h + 3) / 4), pp))
         return run_host_bc1_parts(rgba, blocks, w, h, 8, pp, false, "bc1 encode");
-    return run_host_banded(rgba, blocks, true, w, h, 8,
+    return run_host_banded(rgba, blocks, true, w, h, 1,
                            [&](void *in, void *out, long b0, long b1, void *s) {
                                return qtk::launch_bc1_encode_range((const uint8_t *)in, w, h, pp, (uint8_t *)out, false, b0, b1, s);
                            },
@@ -1063,7 +1082,7 @@ int qt_bc3_encode_host(const uint8_t *rgba, int w, int h, const qt_bc1_params *p
     const qt_bc1_params pp = *p;
     if (qtk::bc1_parts_eligible((long)((w + 3) / 4) * ((h + 3) / 4), pp))
         return run_host_bc1_parts(rgba, blocks, w, h, 16, pp, true, "bc3 encode");
-    return run_host_banded(rgba, blocks, true, w, h, 16,
+    return run_host_banded(rgba, blocks, true, w, h, 3,
                            [&](void *in, void *out, long b0, long b1, void *s) {
                                return qtk::launch_bc1_encode_range((const uint8_t *)in, w, h, pp, (uint8_t *)out, true, b0, b1, s);
                            },
@@ -1075,7 +1094,7 @@ int qt_bc4_encode_host(const uint8_t *rgba, int w, int h, int channel, uint8_t *
     if ((rc = check_dims(w, h)) || (rc = check_channel(channel)) || (rc = check_ptr(rgba, 1, "rgba")) ||
         (rc = check_ptr(blocks, 1, "blocks")))
         return rc;
-    return run_host_banded(rgba, blocks, true, w, h, 8,
+    return run_host_banded(rgba, blocks, true, w, h, 4,
                            [&](void *in, void *out, long b0, long b1, void *s) {
                                return qtk::launch_bc4_encode_range((const uint8_t *)in, w, h, channel, channel, false, (uint8_t *)out, b0, b1, s);
                            },
@@ -1087,7 +1106,7 @@ int qt_bc5_encode_host(const uint8_t *rgba, int w, int h, int c0, int c1, uint8_
     if ((rc = check_dims(w, h)) || (rc = check_channel(c0)) || (rc = check_channel(c1)) ||
         (rc = check_ptr(rgba, 1, "rgba")) || (rc = check_ptr(blocks, 1, "blocks")))
         return rc;
-    return run_host_banded(rgba, blocks, true, w, h, 16,
+    return run_host_banded(rgba, blocks, true, w, h, 5,
                            [&](void *in, void *out, long b0, long b1, void *s) {
                                return qtk::launch_bc4_encode_range((const uint8_t *)in, w, h, c0, c1, true, (uint8_t *)out, b0, b1, s);
                            },
@@ -1110,8 +1129,7 @@ static int decode_host(int fmt, const uint8_t *blocks, int w, int h, int interp,
     if ((rc = check_dims(w, h)) || (rc = check_interp(interp)) || (rc = check_channel(c0)) || (rc = check_channel(c1)) ||
         (rc = check_ptr(blocks, 1, "blocks")) || (rc = check_ptr(rgba, 1, "rgba")))
         return rc;
-    const size_t bsize = (fmt == 3 || fmt == 5) ? 16 : 8;
-    return run_host_banded(blocks, rgba, false, w, h, bsize,
+    return run_host_banded(blocks, rgba, false, w, h, fmt,
                            [&](void *in, void *out, long b0, long b1, void *s) {
                                return qtk::launch_decode_range(fmt, (const uint8_t *)in, w, h, interp, wa, c0, c1, (uint8_t *)out, b0, b1, s);
                            },

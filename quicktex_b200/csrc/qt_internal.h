@@ -140,6 +140,8 @@ int batch_sms();
 extern "C" int qtk_resize_is_small(int w, int h, int dw, int dh);
 // Whether a BC1/BC3 texture of n blocks runs the cooperative encoder on a device whose deferred path starts at defer_min blocks.
 extern "C" int qtk_coop_rule(const qt_bc1_params *p, long n, long defer_min);
+// Whether the host entry points' kernels work on host memory directly for such a texture (fmt 1, 3, 4, 5).
+extern "C" int qtk_host_direct(int encode, int fmt, int w, int h);
 // Graphs that a batch has built (one, and one more for each growth of its queue or of its set of kernels).
 extern "C" size_t qtk_batch_graphs(const qt_batch *b);
 // Pairs of its present graph's kernels of which the second waits for the first.

@@ -53,3 +53,20 @@ def test_coop_rule_on_148_sms():
     assert [_coop(18, i, d - 1, d) for i in range(4)] == [1, 1, 1, 1] and [_coop(18, i, d, d) for i in range(4)] == [1, 1, 0, 1]
     assert [_coop(17, i, 20000, d) for i in range(4)] == [1, 1, 1, 1] and [_coop(17, i, 20001, d) for i in range(4)] == [1, 1, 0, 1]
     assert [_coop(13, i, 5000, d) for i in range(4)] == [1, 1, 0, 1] and _coop(13, 0, 5001, d) == 0 and _coop(12, 0, 100, d) == 0
+
+
+# sizes at which the kernel took longer on host memory than with the copies around it, and at which it was faster
+STAGED = [(0, 1, 8, 24000), (0, 4, 4, 24000), (0, 3, 12, 8000), (0, 1, 33, 7000), (0, 1, 17, 2400), (0, 1, 125, 1500), (0, 4, 191, 1000), (0, 5, 33, 7000),
+          (0, 3, 99, 1200), (1, 5, 500, 508), (1, 5, 12, 12000), (1, 4, 8, 32000), (1, 1, 512, 512), (0, 1, 512, 512), (0, 1, 511, 513)]
+DIRECT = [(0, 1, 256, 256), (0, 1, 401, 399), (0, 1, 510, 334), (0, 3, 128, 128), (0, 5, 129, 127), (0, 1, 64, 64), (0, 1, 63, 61), (0, 1, 7, 5), (0, 4, 250, 250),
+          (1, 5, 480, 528), (1, 5, 500, 200), (1, 5, 501, 500), (1, 4, 12, 8000), (1, 1, 2, 30000), (1, 1, 508, 508), (1, 3, 17, 12000)]
+
+
+@pytest.mark.parametrize("encode,fmt,w,h", STAGED)
+def test_host_textures_with_many_small_pieces_are_staged(encode, fmt, w, h):
+    assert capi.lib().qtk_host_direct(encode, fmt, w, h) == 0
+
+
+@pytest.mark.parametrize("encode,fmt,w,h", DIRECT)
+def test_other_small_host_textures_are_direct(encode, fmt, w, h):
+    assert capi.lib().qtk_host_direct(encode, fmt, w, h) == 1
