@@ -233,6 +233,16 @@ int qtk::check_item_fields(const qt_batch_item &it) {
 }
 
 extern "C" size_t qtk_batch_graphs(const qt_batch *b) { return b->graphs; }
+extern "C" size_t qtk_batch_kernels(const qt_batch *b, unsigned *ctas, unsigned *threads) {
+    size_t n = 0;
+    for (uint32_t left = b->enabled; left; left &= left - 1) {
+        cudaKernelNodeParams np = {};
+        if (cudaGraphKernelNodeGetParams(b->node[__builtin_ctz(left)], &np) != cudaSuccess) return 0;
+        ctas[n] = np.gridDim.x;
+        threads[n++] = np.blockDim.x;
+    }
+    return n;
+}
 extern "C" size_t qtk_batch_edges(const qt_batch *b) {
     size_t n = 0;
     if (b->graph) cudaGraphGetEdges(b->graph, nullptr, nullptr, &n);

@@ -144,6 +144,8 @@ extern "C" int qtk_coop_rule(const qt_bc1_params *p, long n, long defer_min);
 extern "C" int qtk_host_direct(int encode, int fmt, int w, int h);
 // Graphs that a batch has built (one, and one more for each growth of its queue or of its set of kernels).
 extern "C" size_t qtk_batch_graphs(const qt_batch *b);
+// CTAs and threads per CTA of the kernels that its last run launched; their number.
+extern "C" size_t qtk_batch_kernels(const qt_batch *b, unsigned *ctas, unsigned *threads);
 // Pairs of its present graph's kernels of which the second waits for the first.
 extern "C" size_t qtk_batch_edges(const qt_batch *b);
 

@@ -1,6 +1,6 @@
-"""GPU: the grid and CTA size that a batch was given hold for all of its kernels, as the CUDA profiler records them."""
+"""GPU: the grid and CTA size that a batch was given hold for all of its kernels, as they stand in its graph."""
 
-import json
+import ctypes
 
 import numpy as np
 import pytest
@@ -18,22 +18,16 @@ def _jobs():
     return jobs + [Job.encode("bc3", img, 300, 260, level=17), Job.encode("bc4", img, 300, 260, channel=1)]
 
 
-def _kernels(b, jobs, tmp_path):
-    import torch
-    from torch.profiler import ProfilerActivity, profile
-
-    run_jobs(jobs, batch=b)
-    with profile(activities=[ProfilerActivity.CUDA]) as prof:
-        out = run_jobs(jobs, batch=b)
-        torch.cuda.synchronize()
-    path = tmp_path / "trace.json"
-    prof.export_chrome_trace(str(path))
-    ev = [e for e in json.loads(path.read_text())["traceEvents"] if e.get("cat") == "kernel" and "k_batch" in e["name"]]
-    return out, sorted(ev, key=lambda e: e["ts"])
+def _kernels(b, jobs):
+    """The outputs, (CTAs, threads per CTA) of each kernel that the last run launched, and how many of them wait for another."""
+    out = run_jobs(jobs, batch=b)
+    grid, block = ((ctypes.c_uint * 26)() for _ in range(2))
+    n = capi.lib().qtk_batch_kernels(b.handle, grid, block)
+    return out, list(zip(grid[:n], block[:n])), capi.lib().qtk_batch_edges(b.handle)
 
 
 @pytest.mark.parametrize("threads,ctas", [(128, 1), (128, 3), (64, 1), (64, 3), (32, 1), (32, 2), (32, 3)])
-def test_a_limited_grid_holds_for_every_kernel(threads, ctas, tmp_path):
+def test_a_limited_grid_holds_for_every_kernel(threads, ctas):
     import torch
 
     sms = torch.cuda.get_device_properties(0).multi_processor_count
@@ -43,19 +37,16 @@ def test_a_limited_grid_holds_for_every_kernel(threads, ctas, tmp_path):
     try:
         b.set_threads(threads)
         b.set_grid(ctas)
-        out, ev = _kernels(b, jobs, tmp_path)
-        edges = capi.lib().qtk_batch_edges(b.handle)
+        out, kernels, edges = _kernels(b, jobs)
     finally:
         b.close()
     assert out == ref
-    assert len(ev) == 5  # BC4; cooperative; Check2 four-colour; Faster three-colour; Check2 three-colour + black
-    for e in ev:
-        grid, block = (np.prod(e["args"][k]) for k in ("grid", "block"))
-        assert grid * block <= sms * ctas * threads, e["name"]
-    assert edges == len(ev) - 1  # one after the other
+    assert len(kernels) == 5  # BC4; cooperative; Check2 four-colour; Faster three-colour; Check2 three-colour + black
+    assert max(n * t for n, t in kernels) <= sms * ctas * threads
+    assert edges == 4  # one after the other
 
 
-def test_without_a_limit_each_kernel_fills_the_gpu(tmp_path):
+def test_without_a_limit_each_kernel_fills_the_gpu():
     import torch
 
     sms = torch.cuda.get_device_properties(0).multi_processor_count
@@ -65,9 +56,8 @@ def test_without_a_limit_each_kernel_fills_the_gpu(tmp_path):
         for threads, ctas in ((128, 0), (128, 4), (64, 8), (32, 0)):
             b.set_threads(threads)
             b.set_grid(ctas)
-            out, ev = _kernels(b, jobs, tmp_path)
-            assert capi.lib().qtk_batch_edges(b.handle) == 0
-            assert len(ev) == 5 and all(np.prod(e["args"]["grid"]) >= 4 * sms for e in ev)
-            assert {int(np.prod(e["args"]["block"])) for e in ev} == {threads, 128}
+            out, kernels, edges = _kernels(b, jobs)
+            assert edges == 0 and len(kernels) == 5 and min(n for n, _ in kernels) >= 4 * sms
+            assert {t for _, t in kernels} == {threads, 128}
     finally:
         b.close()
