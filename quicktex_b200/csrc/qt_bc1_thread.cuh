@@ -16,6 +16,13 @@
 #define QT_TEXEL_PAD 0
 #endif
 
+// Linkage of the phases that are called. External in the unit that leaves it empty: with `static` the same instructions are
+// scheduled otherwise, and k_bc1_defer at 4096^2, level 13, took 719 us instead of 693 (the call 996 and 971; Nvidia 1045 and 1049).
+// A second unit needs `static`, for the names' sake.
+#ifndef QT_PHASE
+#define QT_PHASE
+#endif
+
 namespace tpb {
 
 constexpr int kThreads = 128;
@@ -110,7 +117,7 @@ __device__ __forceinline__ M metrics_body(bool ignore_black) {
 // their instruction working set small when one kernel serves every setting; the specialised
 // kernels (k_bc1_fast: one selector kind, no EndpointSearch) inline the bodies, which saves
 // the call overhead where the per-block work is small. INL picks one at compile time.
-static __device__ __noinline__ M metrics(bool ignore_black) { return metrics_body(ignore_black); }
+QT_PHASE __device__ __noinline__ M metrics(bool ignore_black) { return metrics_body(ignore_black); }
 template <bool INL> __device__ __forceinline__ M metrics_(bool ignore_black) {
     if constexpr (INL) return metrics_body(ignore_black);
     else return metrics(ignore_black);
@@ -493,7 +500,7 @@ __device__ __forceinline__ int2 find_endpoints_body(const M &m, int mode, bool i
     return make_int2(lo, hi);
 }
 
-static __device__ __noinline__ int2 find_endpoints(const M &m, int mode, bool ignore_black, int power_iters) {
+QT_PHASE __device__ __noinline__ int2 find_endpoints(const M &m, int mode, bool ignore_black, int power_iters) {
     return find_endpoints_body(m, mode, ignore_black, power_iters);
 }
 template <bool INL> __device__ __forceinline__ int2 find_endpoints_(const M &m, int mode, bool ignore_black, int power_iters) {

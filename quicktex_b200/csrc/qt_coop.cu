@@ -2,6 +2,7 @@
 // rows are a bank apart, which the one-block-per-lane kernels do without (level 0 at 4096^2 measured 188 us against 200
 // with them).
 #define QT_TEXEL_PAD 1
+#define QT_PHASE static
 
 #include <cuda_fp16.h>
 
