@@ -115,7 +115,8 @@ int qt_bc3_encode_device(const uint8_t *rgba, int width, int height, const qt_bc
 
 /* No reference counterpart: host memory for texture storage from the library's cache of
  * pinned (page-locked) blocks. The *_host entry points copy pinned buffers with the copy
- * engines directly; pageable buffers go through a pinned staging ring first, which costs
+ * engines directly, or have the kernel of a small texture work on such a block itself;
+ * pageable buffers go through a pinned staging ring first, which costs
  * about as much again on a large texture. A block is page-locked once, when first
  * allocated, and a freed block stays cached for the next allocation of its size class
  * (sizes round up by at most 12.5%; up to 2 GiB stay cached). Blocks under 256 KiB, and
