@@ -261,7 +261,8 @@ __device__ __forceinline__ int2 output_taps_thread(const Scale &S, int o, int32_
 // their share of the vertical sums, all in shared memory; the CTAs then add the shares, each for some of the columns. A
 // row of the horizontal pass is computed by the ~2 output rows that need it; for that the call is one launch without
 // scratch memory: three launches and the allocation take 22 us of host time, one 11, and a chain's small levels have
-// nothing else. G as in k_resample_h.
+// nothing else. G as in k_resample_h. Five CTAs per SM: with the four that 50 registers leave, 85 rows wait for a second wave (23 x 156 ->
+// 2 x 85 12.5 us, with five 8.4).
 constexpr int kSplit = 8;
 struct SmallLayout {  // word offsets in shared memory
     int kk_v, bounds_h, kk_h, rows, share, words;
@@ -277,7 +278,7 @@ struct SmallLayout {  // word offsets in shared memory
 };
 
 template <int G>
-__global__ void __cluster_dims__(kSplit, 1, 1) __launch_bounds__(256) k_resize_small(const uint32_t *__restrict__ src, Scale h, Scale v, uint32_t *__restrict__ dst, SmallLayout L) {
+__global__ void __cluster_dims__(kSplit, 1, 1) __launch_bounds__(256, 5) k_resize_small(const uint32_t *__restrict__ src, Scale h, Scale v, uint32_t *__restrict__ dst, SmallLayout L) {
     extern __shared__ __align__(16) int32_t sm[];  // share is read as int4
     __shared__ int2 bv;
     const cooperative_groups::cluster_group cluster = cooperative_groups::this_cluster();
@@ -354,17 +355,18 @@ __global__ void __cluster_dims__(kSplit, 1, 1) __launch_bounds__(256) k_resize_s
 // Which resizes run as one launch: between separate buffers only (its CTAs read the source while others write the result,
 // where the two passes of the general path have read all of it before the first write), and where the clusters have little to do.
 // Each computes the horizontal taps for itself, and every source row is read by the clusters of the ~2 output rows that need
-// it, so many rows or columns cost more than three launches: up to 128 rows (8 CTAs each: one wave) and 16384
-// texels of result, and 64 K source texels a cluster, which only 8 SMs read. Measured, one launch / general path: 128^2 ->
-// 64^2 6.4 / 13.0 us, 256^2 -> 64^2 8.0 / 12.6, 500^2 -> 125^2 14.6 / 12.6, 512^2 -> 256^2 28.9 / 12.6, 500^2 -> 1000^2
-// 205 / 17; 1024^2 from 300^2 214 / 17; 1086 x 109 -> 66 x 1 (118 K texels a cluster) 33 / 14.4, 510 x 334 -> 7 x 5 (48 K) 17.2 / 16.6.
-constexpr long kSmallTexels = 512L * 512, kSmallRows = 128, kSmallResult = 16384, kSmallRead = 65536;
+// it, so many rows or columns cost more than three launches: up to 128 rows (8 CTAs each: little over a wave), 20480
+// texels of result and 70 K source texels a cluster, which only 8 SMs read; a single texel's launch saves more than that. Measured, one
+// launch / general path: 128^2 -> 64^2 6.7 / 13.0 us, 256^2 -> 64^2 8.0 / 12.6, 500^2 -> 125^2 14.6 / 12.6, 512^2 -> 256^2 28.9 / 12.6,
+// 500^2 -> 1000^2 205 / 17, 300^2 -> 1024^2 214 / 17; 915 x 77 -> 19 x 2 (70,455 texels a cluster) 12.5 / 15.6, 510 x 334 -> 7 x 5 (68,850)
+// 16.6 / 16.6, 500^2 -> 7^2 (72,500) 18.7 / 16.6, 1086 x 109 -> 66 x 1 (118,374) 33 / 14.7; 512^2 -> 1 16.6 / 20.8.
+constexpr long kSmallTexels = 512L * 512, kSmallRows = 128, kSmallResult = 20480, kSmallRead = 71680;
 
 // The result's size first: with it bounded, the layout's and the launch's 32-bit products are in range.
 bool small_resize(const Scale &h, const Scale &v) {
     if ((long)h.in_size * v.in_size > kSmallTexels || v.out_size > kSmallRows || (long)h.out_size * v.out_size > kSmallResult) return false;
     const long rows = v.in_size == v.out_size ? 1 : std::min(v.ksize, v.in_size);
-    return rows * h.in_size <= kSmallRead && (long)SmallLayout(h, v).words * 4 <= 46 * 1024;
+    return (rows * h.in_size <= kSmallRead || h.out_size * v.out_size == 1) && (long)SmallLayout(h, v).words * 4 <= 46 * 1024;
 }
 
 template <int G> void resize_small_g(const uint32_t *in, const Scale &h, const Scale &v, uint32_t *out, cudaStream_t s) {

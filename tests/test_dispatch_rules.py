@@ -28,7 +28,7 @@ def test_resize_with_much_to_do_per_row_is_not_small(w, h, to):
     assert capi.lib().qtk_resize_is_small(w, h, *to) == 0
 
 
-@pytest.mark.parametrize("w,h,to", [(128, 128, (64, 64)), (256, 256, (32, 32)), (500, 500, (62, 62)), (250, 167, (3, 2)), (64, 64, (1, 1))])
+@pytest.mark.parametrize("w,h,to", [(128, 128, (64, 64)), (256, 256, (32, 32)), (500, 500, (62, 62)), (250, 167, (3, 2)), (64, 64, (1, 1)), (512, 512, (1, 1)), (915, 77, (19, 2))])
 def test_small_chains_stay_small(w, h, to):
     assert capi.lib().qtk_resize_is_small(w, h, *to) == 1
 
